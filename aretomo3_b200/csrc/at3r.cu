@@ -4,6 +4,7 @@
 #include "at3r_internal.h"
 #include "fft_host.h"
 #include "recon_kernels.cuh"
+#include "sart_wide.cuh"
 
 #include <cuda_runtime.h>
 #include <dlfcn.h>
@@ -114,6 +115,11 @@ struct at3r_plan {
     int rs_zcrop = 0;                           // radix set of the z-crop kernel (both its lengths)
     size_t smem_rweight = 0, smem_row = 0, smem_zcrop = 0, smem_xc2r = 0;
     int bp_ww_sart = 0, bp_ww_wbp = 0;
+    bool wide = false;   // SART: slices on the lanes (sart_wide.cuh)
+    int fp_seg_rows = 0;                        // its forward projection: volume rows per warp
+    float* d_part = nullptr;                    // sums of the row segments
+    int* d_arrived = nullptr;
+    size_t n_arrived = 0;
     int bp_bulk = 0;   // FP32 back-projection staging by bulk asynchronous copies (AT3R_BP_BULK_STAGING)
     // host path
     float* d_proj_slab[2] = {nullptr, nullptr};
@@ -314,6 +320,76 @@ at3r_status tend(at3r_plan* p, cudaStream_t st, int kind, double bytes, double u
         if (r_ != AT3R_OK) return r_;                                  \
     } while (0)
 
+// A SART slab on the slice-group kernels of sart_wide.cuh, G = LP * NS slices
+// per group.
+template <int LP, int NS>
+at3r_status run_sart_wide(at3r_plan* p, const float* proj, size_t tilt_stride, int proj_y0, int S, float* vol,
+                          cudaStream_t st)
+{
+    constexpr int G = LP * NS;
+    const int T = p->T, N = p->N, Nx = p->Nx, Nz = p->Nz, SG = (S + G - 1) / G;
+    const double f4 = 4.0, vox = (double)S * Nx * Nz, upd = 2 * f4;
+    float* raw = static_cast<float*>(p->d_raw);
+    float* dif = static_cast<float*>(p->d_diff);
+    float* w = reinterpret_cast<float*>(p->d_w);
+    AT3R_CUDA(cudaMemsetAsync(p->d_flags, 0, sizeof(int) * SG * G, st));
+    TB(p, st);
+    k_gather_wide<G><<<dim3((N + 31) / 32, T, SG), 256, 0, st>>>(proj, tilt_stride, p->nx, proj_y0, p->d_cs, T, N, Nz, S,
+                                                                 raw, p->d_flags);
+    TE(p, st, KK_GATHER, 2 * f4 * S * T * N, (double)S * T * N);
+    AT3R_CUDA(cudaMemsetAsync(w, 0, sizeof(float) * (size_t)SG * G * Nx * Nz, st));
+    BpwArgs b{};
+    b.cs = p->d_cs; b.vol = w; b.flags = p->d_flags; b.T = T; b.N = N; b.Nx = Nx; b.Nz = Nz;
+    const dim3 bgrid((Nx + bpw_tile_x<LP>() - 1) / bpw_tile_x<LP>(), (Nz + BPW_TILE_Z - 1) / BPW_TILE_Z, SG);
+    // first back-projection: all tilts, relax 1 (CTomoSart.cpp:68-69)
+    b.sino = raw; b.t0 = 0; b.t1 = T; b.relax = 1.f; b.low_bit = kFlagRawLow;
+    TB(p, st);
+    k_bp_wide<LP, NS><<<bgrid, WIDE_THREADS, bpw_smem<LP, NS>(), st>>>(b);
+    TE(p, st, KK_BP_SART, f4 * S * (double)T * N + upd * vox, vox * T);
+    b.sino = dif; b.relax = p->relax; b.low_bit = kFlagDiffLow;
+    FpwArgs f{};
+    f.vol = w; f.raw = raw; f.diff = dif; f.cs = p->d_cs; f.flags = p->d_flags;
+    f.Nx = Nx; f.Nz = Nz; f.S = S; f.T = T; f.N = N;
+    f.part = p->d_part; f.arrived = p->d_arrived; f.seg_rows = p->fp_seg_rows;
+    const int blocks = (N + FPW_CTA_RAYS - 1) / FPW_CTA_RAYS, segs = (Nz + f.seg_rows - 1) / f.seg_rows;
+    AT3R_CUDA(cudaMemsetAsync(p->d_arrived, 0, sizeof(int) * p->n_arrived, st));
+    for (int it = 0; it < p->g.iterations; it++) {
+        for (size_t s = 0; s < p->sub_start.size(); s++) {
+            const int t0 = p->sub_start[s] + p->g.start_tilt, nt = p->sub_size[s];
+            if (nt <= 0) continue;
+            double samples = 0;
+            for (int t = t0; t < t0 + nt; t++) samples += (double)p->ray_len[t];
+            f.rf = p->g.compute_rfactor ? p->d_rf + 2 * it : nullptr;
+            f.t0 = t0; f.nt = nt;
+            TB(p, st);
+            k_fp_wide<G><<<dim3(blocks * nt, segs, SG), FPW_THREADS, Fpw<G>::SMEM, st>>>(f);
+            TE(p, st, KK_FP_DIFF, f4 * vox + 2.0 * f4 * S * nt * N, samples * N * S);
+            b.t0 = t0; b.t1 = t0 + nt;
+            TB(p, st);
+            k_bp_wide<LP, NS><<<bgrid, WIDE_THREADS, bpw_smem<LP, NS>(), st>>>(b);
+            TE(p, st, KK_BP_SART, f4 * S * (double)nt * N + upd * vox, vox * nt);
+        }
+    }
+    TB(p, st);
+    k_ungroup_wide<G><<<dim3((Nx + 31) / 32, Nz, SG), 256, 0, st>>>(w, vol, Nx, Nz, S);
+    TE(p, st, KK_UNGROUP, 2 * f4 * vox, vox);
+    return AT3R_OK;
+}
+
+// The empty-voxel fill that ends a SART slab (CTomoSart.cpp:88); only flagged slices do work.
+at3r_status run_fill(at3r_plan* p, int S, float* vol, cudaStream_t st)
+{
+    const int Nx = p->Nx, Nz = p->Nz;
+    const int fb = std::max(1, std::min((Nx * Nz + 255) / 256, (8 * 148 + S - 1) / S));
+    TB(p, st);
+    k_fill_mark<<<dim3(fb, S), 256, 0, st>>>(vol, Nx, Nz, p->d_flags, p->fill_seed, p->d_seen);
+    TE(p, st, KK_FILL, 4.0 * S, 0);
+    TB(p, st);
+    k_fill_finish<<<S, 512, 0, st>>>(vol, Nx, Nz, p->d_flags, p->d_seen);
+    TE(p, st, KK_FILL, 4.0 * S, 0);
+    return AT3R_OK;
+}
+
 // One slab of slices [y0, y0 + S): proj points at tilt 0 row 0 of a
 // [T][rows][nx] block whose row `proj_y0` is slice y0; vol points at the
 // slab's first output slice.
@@ -334,6 +410,15 @@ at3r_status run_slab_t(at3r_plan* p, const float* proj, size_t tilt_stride, int 
     const int T = p->T, N = p->N, Nx = p->Nx, Nz = p->Nz, KX = p->KX;
     const double f4 = 4.0, vox = (double)S * Nx * Nz;
     const int SG = (S + SB - 1) / SB;   // slice groups: each thread carries SB slices
+    if (p->wide) {   // (FP32 only)
+        at3r_status rc;
+        switch (wide_group(S)) {
+            case 64: rc = run_sart_wide<8, 8>(p, proj, tilt_stride, proj_y0, S, vol, st); break;
+            case 32: rc = run_sart_wide<8, 4>(p, proj, tilt_stride, proj_y0, S, vol, st); break;
+            default: rc = run_sart_wide<4, 4>(p, proj, tilt_stride, proj_y0, S, vol, st); break;
+        }
+        return rc != AT3R_OK ? rc : run_fill(p, S, vol, st);
+    }
     AT3R_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * S, st));
     if (p->g.method == AT3R_SART) {
         TB(p, st);
@@ -392,15 +477,7 @@ at3r_status run_slab_t(at3r_plan* p, const float* proj, size_t tilt_stride, int 
         k_ungroup<<<dim3((unsigned)(((size_t)Nx * Nz + 255) / 256), SG), 256, 0, st>>>(p->d_w, vol, S,
                                                                                        (size_t)Nx * Nz);
         TE(p, st, KK_UNGROUP, 2 * f4 * vox, vox);
-        // the empty-voxel fill (CTomoSart.cpp:88); only flagged slices do work
-        const int fb = std::max(1, std::min((Nx * Nz + 255) / 256, (8 * 148 + S - 1) / S));
-        TB(p, st);
-        k_fill_mark<<<dim3(fb, S), 256, 0, st>>>(vol, Nx, Nz, p->d_flags, p->fill_seed, p->d_seen);
-        TE(p, st, KK_FILL, f4 * S, 0);
-        TB(p, st);
-        k_fill_finish<<<S, 512, 0, st>>>(vol, Nx, Nz, p->d_flags, p->d_seen);
-        TE(p, st, KK_FILL, f4 * S, 0);
-        return AT3R_OK;
+        return run_fill(p, S, vol, st);
     }
     // WBP
     TB(p, st);
@@ -528,15 +605,65 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
 
 at3r_status at3r_plan_create(const at3r_geom* g, at3r_plan** out) { return plan_create_impl(g, nullptr, out); }
 
+// SART on slice groups (sart_wide.cuh): FP32 series whose rows fill the groups.  Full
+// groups take 0.62 (4096 wide) to 0.72 (1024 wide) of the four-slice kernels' time, so they
+// pay as long as filling up costs less than 1.3; the 16-bit forms of the four-slice kernels
+// are as fast as full groups (2048 x 96 x 600: 55.9 ms against 54.7; 925 x 131 x 221:
+// 15.5 against 17.1) and stay.  It follows the series, not the slab, so that a slab size
+// never changes a result.
+constexpr double kWideFill = 1.3;
+static bool sart_wide(const at3r_geom* g)
+{
+    return g->method == AT3R_SART && g->storage == AT3R_STORE_F32 && wide_cost(g->ny) <= kWideFill * g->ny;
+}
+
+// The most tilts of a subset.
+static size_t wide_subset(const at3r_geom* g)
+{
+    return std::max(1, (g->num_tilts + g->subsets - 1) / std::max(1, g->subsets));
+}
+// Volume rows per warp of the forward projection: enough segments that one
+// subset's projection gives every SM two rounds of its eight warps, and at most
+// 320 rows, so that the concurrent walks stay within what L2 holds of the
+// volume.  It follows the series, not the slab (the segments' sums are part of a result).
+static int wide_seg_rows(const at3r_geom* g)
+{
+    const long N = g->nx & ~1, warps = (N + 15) / 16 * (long)wide_subset(g) * ((g->ny + 63) / 64);
+    const long segs = std::max((long)(g->vol_z + 319) / 320, std::min((long)(2 * 8 * 148 + warps - 1) / warps, (long)g->vol_z / 24));
+    return (int)((g->vol_z + std::max(segs, 1L) - 1) / std::max(segs, 1L));
+}
+// Counters of the segments: one per group of 16 or more slices, tilt and 16 or more rays.
+static size_t wide_arrived(const at3r_geom* g, int slices)
+{
+    return (size_t)((slices + 15) / 16) * wide_subset(g) * (size_t)(((g->nx & ~1) + 15) / 16);
+}
+
+// Workspace bytes one slice adds: SART two staged rows per tilt, the working
+// volume and, in the 16-bit forms, its 16-bit copy; WBP the filtered rows, the
+// 2x grid and the row spectra.
+static size_t slice_bytes(const at3r_geom* g)
+{
+    const size_t T = g->n_tilts, N = g->nx & ~1, Nz = g->vol_z, KX = N / 2 + 1;
+    const size_t esz = g->storage == AT3R_STORE_F32 ? 4 : 2;
+    if (g->method == AT3R_SART)
+    {
+        if (sart_wide(g))   // with the segments' sums and counters
+            return 8 * T * N + 4 * N * Nz +
+                   wide_subset(g) * ((Nz + wide_seg_rows(g) - 1) / wide_seg_rows(g) * N * 4 + (N + 15) / 16);
+        return 2 * T * N * esz + 4 * N * Nz + (esz < 4 ? 2 * N * Nz + 4 * T : 0);
+    }
+    return T * N * sizeof(float) + 16 * N * Nz + 2 * Nz * KX * sizeof(float2);
+}
+
 // Default slab (slices per launch).  SART: enough slice groups that one
 // subset's forward projection (grid ceil(N/256) x tilts x groups) spans about
 // 16 waves of 6 CTAs on every SM — measured on B200, the SART rate keeps
 // rising with the slab up to the whole series (1024 x 1024 x 61: 37.9
 // GVoxel*tilt/s at 58 slices, 55.2 at 1024) — with the workspace capped at
 // 8 GB.  WBP: a 256 MB workspace (larger slabs gain under 3 %).
-// per_slice: workspace bytes one slice adds.
-int default_slab(const at3r_geom* g, size_t per_slice, int sms)
+int default_slab(const at3r_geom* g, int sms)
 {
+    const size_t per_slice = slice_bytes(g);
     long S;
     if (g->method == AT3R_SART) {
         const long N = g->nx & ~1;
@@ -549,6 +676,7 @@ int default_slab(const at3r_geom* g, size_t per_slice, int sms)
         S = (long)(((size_t)256 << 20) / std::max<size_t>(per_slice, 1));
     }
     S = std::max(S, 8L);
+    if (sart_wide(g) && S > 64) S -= S % 64;   // whole slice groups
     return (int)std::min<long>(S, g->ny);
 }
 
@@ -560,18 +688,13 @@ size_t at3r_plan_estimate_bytes(const at3r_geom* g)
     if (!g || g->nx < 1 || g->ny < 1 || g->n_tilts < 1 || g->vol_z < 1) return 0;
     const size_t T = g->n_tilts, N = g->nx & ~1, Nx = N, Nz = g->vol_z, KX = Nx / 2 + 1, nx = g->nx;
     const size_t esz = g->storage == AT3R_STORE_F32 ? 4 : 2;
-    size_t per_slice, tables = 0;
-    if (g->method == AT3R_SART) {
-        per_slice = 2 * T * N * esz + 4 * Nx * Nz + (esz < 4 ? 2 * Nx * Nz + 4 * T : 0);
-    } else {
-        per_slice = T * N * sizeof(float) + 16 * Nx * Nz + 2 * Nz * KX * sizeof(float2);
-        tables = 4 * sizeof(float2) * 4 * (N + 2 * Nx + 3 * Nz + Nx);   // Bluestein can take 4x the length
-    }
-    size_t slab = g->slab_slices > 0 ? (size_t)g->slab_slices : (size_t)default_slab(g, per_slice, 148);
+    // Bluestein can take 4x the length
+    const size_t tables = g->method == AT3R_SART ? 0 : 4 * sizeof(float2) * 4 * (N + 2 * Nx + 3 * Nz + Nx);
+    size_t slab = g->slab_slices > 0 ? (size_t)g->slab_slices : (size_t)default_slab(g, 148);
     slab = std::min<size_t>(slab, (size_t)g->ny);
     size_t work;
     if (g->method == AT3R_SART)
-        work = (slab + 7) * (2 * T * N * esz + 4 * Nx * Nz + (esz < 4 ? 2 * Nx * Nz + T * 4 : 0)) + slab * 8;
+        work = (sart_wide(g) ? wide_slices((int)slab) : slab + 7) * (slice_bytes(g) + 4) + slab * 8;
     else   // two lanes of slab workspace when the series has more than one slab (device path)
         work = (slab < (size_t)g->ny ? 2 : 1) *
                slab * (T * N * esz + 16 * Nx * Nz + 2 * Nz * KX * sizeof(float2) + (esz < 4 ? T * 4 : 0) + 4);
@@ -589,17 +712,13 @@ size_t at3r_estimate_resident_bytes(const at3r_geom* g, int* slab_out)
     if (!g || g->nx < 1 || g->ny < 1 || g->n_tilts < 1 || g->vol_z < 1) return 0;
     const size_t T = g->n_tilts, N = g->nx & ~1, Nx = N, Nz = g->vol_z, KX = Nx / 2 + 1, nx = g->nx, ny = g->ny;
     const size_t esz = g->storage == AT3R_STORE_F32 ? 4 : 2;
-    size_t per_slice, tables = 0, work;
-    if (g->method == AT3R_SART) {
-        per_slice = 2 * T * N * esz + 4 * Nx * Nz + (esz < 4 ? 2 * Nx * Nz + 4 * T : 0);
-    } else {
-        per_slice = T * N * sizeof(float) + 16 * Nx * Nz + 2 * Nz * KX * sizeof(float2);
-        tables = 4 * sizeof(float2) * 4 * (N + 2 * Nx + 3 * Nz + Nx);
-    }
-    size_t slab = g->slab_slices > 0 ? (size_t)g->slab_slices : (size_t)default_slab(g, per_slice, 148);
+    // Bluestein can take 4x the length
+    const size_t tables = g->method == AT3R_SART ? 0 : 4 * sizeof(float2) * 4 * (N + 2 * Nx + 3 * Nz + Nx);
+    size_t slab = g->slab_slices > 0 ? (size_t)g->slab_slices : (size_t)default_slab(g, 148);
     slab = std::min<size_t>(slab, ny);
+    size_t work;
     if (g->method == AT3R_SART)
-        work = (slab + 7) * (2 * T * N * esz + 4 * Nx * Nz + (esz < 4 ? 2 * Nx * Nz + T * 4 : 0)) + slab * 8;
+        work = (sart_wide(g) ? wide_slices((int)slab) : slab + 7) * (slice_bytes(g) + 4) + slab * 8;
     else
         work = slab * (T * N * esz + 16 * Nx * Nz + 2 * Nz * KX * sizeof(float2) + (esz < 4 ? T * 4 : 0) + 4);
     if (slab_out) *slab_out = (int)slab;
@@ -675,8 +794,8 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
         return fail(set_err(AT3R_ERR_CUDA, "geometry upload failed"));
 
     const size_t T = p->T, N = p->N, Nx = p->Nx, Nz = p->Nz, KX = p->KX;
-    size_t per_slice;
     if (g->method == AT3R_SART) {
+        p->wide = sart_wide(g);
         p->relax = g->relax > 0.f ? g->relax : 1.0f / (float)g->subsets;
         // AreTomo/Util/CSplitItems.cpp:25-48
         const int n = g->num_tilts, k = g->subsets;
@@ -690,7 +809,15 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
                                (const void*)k_bp<0, __nv_bfloat16, __nv_bfloat16, true>})
             if ((rc = set_smem(fn, bp_smem(0)))) return fail(rc);
         if (p->bp_bulk && (rc = set_smem((const void*)k_bp<0, float, float, true, true>, bp_smem(1)))) return fail(rc);
-        per_slice = 2 * T * N * p->esz + 4 * Nx * Nz + (p->esz < 4 ? 2 * Nx * Nz + 4 * T : 0);
+        if (p->wide) {
+            for (auto& f : {std::make_pair((const void*)k_fp_wide<64>, Fpw<64>::SMEM),
+                            std::make_pair((const void*)k_fp_wide<32>, Fpw<32>::SMEM),
+                            std::make_pair((const void*)k_fp_wide<16>, Fpw<16>::SMEM),
+                            std::make_pair((const void*)k_bp_wide<8, 8>, bpw_smem<8, 8>()),
+                            std::make_pair((const void*)k_bp_wide<8, 4>, bpw_smem<8, 4>()),
+                            std::make_pair((const void*)k_bp_wide<4, 4>, bpw_smem<4, 4>())})
+                if ((rc = set_smem(f.first, f.second))) return fail(rc);
+        }
     } else {
         if (g->c2r == AT3R_C2R_MATCH_CUFFT) {
             bool measured = false;
@@ -754,16 +881,28 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
         }
         if ((rc = dalloc(p, &p->d_h, h.size()))) return fail(rc);
         cudaMemcpy(p->d_h, h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice);
-        per_slice = T * N * sizeof(float) + 16 * Nx * Nz + 2 * Nz * KX * sizeof(float2);
     }
 
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
-    int slab = g->slab_slices > 0 ? g->slab_slices : default_slab(g, per_slice, sms);
+    int slab = g->slab_slices > 0 ? g->slab_slices : default_slab(g, sms);
     p->slab = std::min(slab, p->ny);
     p->slab_cap = p->slab;
     const size_t S = p->slab;
-    if (g->method == AT3R_SART) {
+    if (p->wide) {
+        const size_t W = wide_slices(p->slab);
+        if ((rc = dalloc_bytes(p, &p->d_raw, W * T * N * sizeof(float)))) return fail(rc);
+        if ((rc = dalloc_bytes(p, &p->d_diff, W * T * N * sizeof(float)))) return fail(rc);
+        if ((rc = dalloc_bytes(p, reinterpret_cast<void**>(&p->d_w), sizeof(float) * W * Nx * Nz))) return fail(rc);
+        if ((rc = dalloc(p, &p->d_flags, W))) return fail(rc);
+        if ((rc = dalloc(p, &p->d_rf, 2 * (size_t)std::max(1, g->iterations)))) return fail(rc);
+        p->fp_seg_rows = wide_seg_rows(g);
+        const size_t nt = wide_subset(g), segs = (Nz + p->fp_seg_rows - 1) / p->fp_seg_rows;
+        p->n_arrived = wide_arrived(g, (int)W);
+        if ((rc = dalloc(p, &p->d_part, std::max<size_t>(segs * nt * N * W, 4)))) return fail(rc);
+        if ((rc = dalloc(p, &p->d_arrived, p->n_arrived))) return fail(rc);
+        p->h_rf.assign(2 * std::max(1, g->iterations), 0.0);
+    } else if (g->method == AT3R_SART) {
         if ((rc = dalloc_bytes(p, &p->d_raw, S * T * N * p->esz))) return fail(rc);
         if ((rc = dalloc_bytes(p, &p->d_diff, S * T * N * p->esz))) return fail(rc);
         if (g->storage != AT3R_STORE_F32) {
@@ -793,7 +932,7 @@ void at3r_plan_destroy(at3r_plan* p)
     // like cudaFree, wait for work that may still use the plan's memory
     if (p->pooled) cudaDeviceSynchronize();
     for (void* ptr : {(void*)p->d_cs, (void*)p->d_seen, (void*)p->d_raw, (void*)p->d_diff, (void*)p->d_scale, (void*)p->d_shadow,
-                      (void*)p->d_w,
+                      (void*)p->d_w, (void*)p->d_part, (void*)p->d_arrived,
                       (void*)p->d_flags, (void*)p->d_rf, (void*)p->d_h, (void*)p->d_filt, (void*)p->d_g2,
                       (void*)p->d_y})
         dfree(p, ptr);

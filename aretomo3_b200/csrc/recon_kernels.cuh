@@ -167,6 +167,8 @@ __device__ __forceinline__ float row_scale(float absmax) { return absmax > 0.f ?
 constexpr int kFlagVolEmpty = 1;    // the volume holds a -1e30 voxel (AreTomo's "empty")
 constexpr int kFlagRawLow = 2;      // the staged sinogram holds values <= kLowValue
 constexpr int kFlagDiffLow = 4;     // the residual holds values <= kLowValue
+constexpr int kFlagRawSpecial = 32, kFlagDiffSpecial = 64, kFlagVolSpecial = 128;   // see sart_wide.cuh
+constexpr int kFlagsReported = 31;  // the bits of the run summary
 constexpr float kLowValue = -5.0e9f;  // far from any lerp of values above it reaching -1e10
 
 // y-slices one thread carries: every slice has the same geometry (single
@@ -1368,7 +1370,7 @@ __global__ void __launch_bounds__(512) k_fill_finish(float* __restrict__ vol, in
 {
     const int ys = blockIdx.x, tid = threadIdx.x;
     const int f = flags[ys];
-    if (tid == 0 && seen) atomicOr(seen, f);
+    if (tid == 0 && seen) atomicOr(seen, f & kFlagsReported);
     if ((f & kFlagVolEmpty) == 0) return;
     const int n = Nx * Nz;
     float* v = vol + (size_t)ys * n;

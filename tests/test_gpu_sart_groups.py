@@ -1,0 +1,77 @@
+"""GPU: the SART kernels that put a slice group (16, 32 or 64 rows) on the lanes
+(FP32 series whose rows fill the groups), at the sizes where they can go wrong,
+against the FP64 oracle.
+
+Tolerance: a value is a few thousand FP32 multiply-adds, so its relative error
+is about sqrt(n) * 2^-24 ~ 4e-6 of the volume's scale; 2e-5 leaves the
+few iterations' worth of room."""
+import numpy as np
+import pytest
+
+from oracle_lib import rel_l2, sart
+
+pytestmark = pytest.mark.gpu
+
+TOL = 2e-5
+
+
+def _series(nx, ny, tilts, vol_z, seed):
+    from aretomo3_b200 import synth
+    ph = synth.Phantom(seed=seed, n_ellipsoids=30, axis_min=3, axis_max=14, n_beads=3, bead_radius=2,
+                       noise_kind=synth.NOISE_POISSON, noise_param=50.0)
+    return synth.make_tilt_series(nx, ny, tilts, vol_z, ph)
+
+
+def _run(frames, tilts, vol_z, **kw):
+    from aretomo3_b200 import recon
+    T, ny, nx = frames.shape
+    plan = recon.Plan(nx, ny, tilts, vol_z, method=recon.SART, fill_seed=3, **kw)
+    try:
+        vol = np.empty(plan.volume_shape, np.float32)
+        plan.run_host([frames[t] for t in range(T)], [vol[y] for y in range(ny)])
+        return vol, plan.flags_seen()
+    finally:
+        plan.close()
+
+
+# rows that fill and part-fill the groups, and rows that do not use them; widths that fill no
+# ray block or voxel tile, down to the narrowest; odd thicknesses; tilts from flat to beyond the
+# blocked windows (80+ degrees)
+@pytest.mark.parametrize("nx,ny,nz,lim", [(64, 8, 24, 60), (65, 32, 31, 60), (34, 27, 17, 50), (130, 50, 40, 66),
+                                          (48, 33, 2, 60), (4, 64, 9, 45), (6, 30, 5, 60), (97, 91, 50, 60),
+                                          (250, 30, 75, 85), (40, 50, 200, 75)])
+def test_sizes_vs_oracle(nx, ny, nz, lim):
+    tilts = np.linspace(-lim, lim, 23).astype(np.float32)
+    f = _series(nx, ny, tilts, nz, seed=nx + ny)
+    vol, seen = _run(f, tilts, nz, iterations=3, subsets=4)
+    assert not seen & 16, "a bulk copy did not arrive"
+    assert rel_l2(vol, sart(f, tilts, nz, 0, tilts.size, 3, 4)) < TOL
+
+
+@pytest.mark.parametrize("storage", [0, 1, 2])
+def test_slab_size_does_not_change_a_result(storage):
+    """Groups of 16, 32 and 64 rows, whole and part-filled, give the same bits."""
+    tilts = np.linspace(-60, 60, 21).astype(np.float32)
+    f = _series(140, 64, tilts, 37, seed=5)
+    ref, _ = _run(f, tilts, 37, iterations=2, subsets=3, storage=storage)
+    for slab in (1, 5, 16, 20, 40, 63):
+        vol, _ = _run(f, tilts, 37, iterations=2, subsets=3, storage=storage, slab_slices=slab)
+        assert np.array_equal(vol, ref), slab
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf, 1e35, -1e30, -3e9])
+def test_an_unusual_row_leaves_the_others_alone(bad):
+    """Rows with NaN, infinite, huge, missing or near-missing pixels take the
+    per-sample paths; the other rows of their group keep their bits."""
+    tilts = np.linspace(-60, 60, 21).astype(np.float32)
+    f = _series(96, 30, tilts, 32, seed=11)
+    ref, _ = _run(f, tilts, 32, iterations=2, subsets=4)
+    g = f.copy()
+    g[3, 5, 40:44] = bad
+    g[10, 13, 7] = bad
+    vol, _ = _run(g, tilts, 32, iterations=2, subsets=4)
+    same = [y for y in range(30) if y not in (5, 13)]
+    assert np.array_equal(vol[same], ref[same])
+    assert not np.array_equal(vol[5], ref[5])
+    if bad in (-1e30, -3e9):
+        assert rel_l2(vol, sart(g, tilts, 32, 0, 21, 2, 4)) < 1e-4
