@@ -5,6 +5,7 @@
 #include "fft_host.h"
 #include "recon_kernels.cuh"
 #include "sart_wide.cuh"
+#include "wbp_wave.cuh"
 
 #include <cuda_runtime.h>
 #include <dlfcn.h>
@@ -114,13 +115,12 @@ struct at3r_plan {
     int b_rweight = 1, b_row = 1, b_xc2r = 1;   // sequences per CTA of the row FFT kernels
     int rs_zcrop = 0;                           // radix set of the z-crop kernel (both its lengths)
     size_t smem_rweight = 0, smem_row = 0, smem_zcrop = 0, smem_xc2r = 0;
-    int bp_ww_sart = 0, bp_ww_wbp = 0;
+    int bp_ww_sart = 0;
     bool wide = false;   // SART: slices on the lanes (sart_wide.cuh)
     int fp_seg_rows = 0;                        // its forward projection: volume rows per warp
     float* d_part = nullptr;                    // sums of the row segments
     int* d_arrived = nullptr;
     size_t n_arrived = 0;
-    int bp_bulk = 0;   // FP32 back-projection staging by bulk asynchronous copies (AT3R_BP_BULK_STAGING)
     // host path
     float* d_proj_slab[2] = {nullptr, nullptr};
     float* d_vol_slab[2] = {nullptr, nullptr};
@@ -229,19 +229,6 @@ int bp_window(int tx, int tz, double scale, const std::vector<float>& cs, int T)
 }
 
 // tilts are staged in chunks, so the window buffer does not grow with the tilt count
-// dynamic shared memory of a back-projection launch (bulk: the bulk-copy
-// staging's raw rows and mbarrier on top)
-size_t bp_smem(int bulk) { return bp_smem_bytes(bulk); }
-
-// Back-projection window staging by bulk asynchronous copies (FP32 storage,
-// N a multiple of 4): off unless AT3R_BP_BULK_STAGING=1 at plan creation; an
-// alternative to the load path, kept for comparison.
-bool bp_bulk_from_env()
-{
-    const char* e = std::getenv("AT3R_BP_BULK_STAGING");
-    return e && e[0] == '1';
-}
-
 // Threads of a row / column FFT launch: 1024 when two CTAs' shared memory
 // would not fit one SM (so one CTA holds 32 warps) and the radix set allows.
 int fft_threads(int rs, size_t smem)
@@ -390,6 +377,14 @@ at3r_status run_fill(at3r_plan* p, int S, float* vol, cudaStream_t st)
     return AT3R_OK;
 }
 
+WbpBpArgs wbp_args(const at3r_plan* p, int S, const void* filt, const float* scale, const int* flags, float* g2)
+{
+    WbpBpArgs a{};
+    a.sino = filt; a.scale = scale; a.cs = p->d_cs; a.flags = flags; a.seen = p->d_seen; a.out = g2;
+    a.T = p->T; a.N = p->N; a.GX = 2 * p->Nx; a.GZ = 2 * p->Nz; a.S = S;
+    return a;
+}
+
 // One slab of slices [y0, y0 + S): proj points at tilt 0 row 0 of a
 // [T][rows][nx] block whose row `proj_y0` is slice y0; vol points at the
 // slab's first output slice.
@@ -434,24 +429,15 @@ at3r_status run_slab_t(at3r_plan* p, const float* proj, size_t tilt_stride, int 
         BpArgs a{};
         a.T = T; a.N = N; a.cs = p->d_cs; a.GX = Nx; a.GZ = Nz; a.S = S;
         a.out = reinterpret_cast<float*>(p->d_w); a.out_slice = (size_t)Nx * Nz; a.ww = p->bp_ww_sart;
-        a.flags = p->d_flags; a.seen = p->d_seen; a.bulk = p->bp_bulk;
+        a.flags = p->d_flags; a.seen = p->d_seen;
         a.scale = p->d_scale; a.shadow = p->d_shadow;
         const dim3 bgrid = bp_paired<VT>()
                                ? dim3(2 * ((Nx + BP_TX - 1) / BP_TX), (Nz + BP_TZ - 1) / BP_TZ, (SG + 1) / 2)
                                : dim3((Nx + BP_TX - 1) / BP_TX, (Nz + BP_TZ - 1) / BP_TZ, SG);
-        auto bp_launch = [&](int nt_) {
-            if constexpr (std::is_same<ST, float>::value) {
-                if (a.bulk) {
-                    k_bp<0, ST, VT, true, true><<<bgrid, BP_THREADS, bp_smem(1), st>>>(a);
-                    return;
-                }
-            }
-            k_bp<0, ST, VT, true><<<bgrid, BP_THREADS, bp_smem(0), st>>>(a);
-        };
         // first back-projection: all tilts, relax 1 (CTomoSart.cpp:68-69)
         a.sino = raw; a.t0 = 0; a.t1 = T; a.relax = 1.f; a.low_bit = kFlagRawLow;
         TB(p, st);
-        bp_launch(T);
+        k_bp<ST, VT, true><<<bgrid, BP_THREADS, bp_smem_bytes(), st>>>(a);
         TE(p, st, KK_BP_SART, es * S * (double)T * N + (2 * f4 + (vs < 4 ? vs : 0)) * vox, vox * T);
         a.sino = dif; a.relax = p->relax; a.low_bit = kFlagDiffLow;
         for (int it = 0; it < p->g.iterations; it++) {
@@ -469,7 +455,7 @@ at3r_status run_slab_t(at3r_plan* p, const float* proj, size_t tilt_stride, int 
                 TE(p, st, KK_FP_DIFF, vs * vox + 2.0 * es * S * nt * N, samples * N * S);
                 a.t0 = t0; a.t1 = t0 + nt;
                 TB(p, st);
-                bp_launch(nt);
+                k_bp<ST, VT, true><<<bgrid, BP_THREADS, bp_smem_bytes(), st>>>(a);
                 TE(p, st, KK_BP_SART, es * S * (double)nt * N + (2 * f4 + (vs < 4 ? vs : 0)) * vox, vox * nt);
             }
         }
@@ -488,20 +474,12 @@ at3r_status run_slab_t(at3r_plan* p, const float* proj, size_t tilt_stride, int 
                                                                    scale, flags);
     });
     TE(p, st, KK_RWEIGHT, (f4 + es) * S * T * N, (double)S * T * N);
-    BpArgs a{};
-    a.sino = filt; a.scale = scale; a.shadow = nullptr; a.T = T; a.N = N; a.t0 = 0; a.t1 = T; a.cs = p->d_cs;
-    a.GX = 2 * Nx; a.GZ = 2 * Nz; a.S = S; a.relax = 1.f; a.out = g2; a.out_slice = (size_t)4 * Nx * Nz;
-    a.ww = p->bp_ww_wbp; a.flags = flags; a.seen = p->d_seen; a.low_bit = kFlagRawLow; a.bulk = p->bp_bulk;
+    const WbpBpArgs a = wbp_args(p, S, filt, scale, flags, g2);
     TB(p, st);
-    const dim3 wgrid((2 * Nx + BP_TX - 1) / BP_TX, (2 * Nz + BP_TZ - 1) / BP_TZ, SG);
-    bool launched = false;
-    if constexpr (std::is_same<ST, float>::value) {
-        if (a.bulk) {
-            k_bp<1, ST, float, false, true><<<wgrid, BP_THREADS, bp_smem(1), st>>>(a);
-            launched = true;
-        }
-    }
-    if (!launched) k_bp<1, ST, float, false><<<wgrid, BP_THREADS, bp_smem(0), st>>>(a);
+    const dim3 wgrid((2 * Nx + WBP_T - 1) / WBP_T, (2 * Nz + WBP_T - 1) / WBP_T, (S + 7) / 8);
+    // eight slices a thread share each position and weight; a slab of four or fewer takes the four-slice form
+    if (S > 4) k_bp_wbp<ST, 8><<<wgrid, WBP_THREADS, wbp_bp_smem<8>(), st>>>(a);
+    else k_bp_wbp<ST, 4><<<wgrid, WBP_THREADS, wbp_bp_smem<4>(), st>>>(a);
     TE(p, st, KK_BP_WBP, es * S * (double)T * N + f4 * 4 * vox, 4 * vox * T);
     TB(p, st);
     dispatch_rs(p->f2x.rs, [&](auto R) {
@@ -676,6 +654,7 @@ int default_slab(const at3r_geom* g, int sms)
         S = (long)(((size_t)256 << 20) / std::max<size_t>(per_slice, 1));
     }
     S = std::max(S, 8L);
+    if (g->method == AT3R_WBP) S -= S % 8;         // whole groups of eight slices (wbp_bp.cuh)
     if (sart_wide(g) && S > 64) S -= S % 64;   // whole slice groups
     return (int)std::min<long>(S, g->ny);
 }
@@ -769,7 +748,6 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
     p->g.tilts_deg = p->tilts.data();
     p->nx = g->nx; p->ny = g->ny; p->T = g->n_tilts;
     p->fill_seed = g->fill_seed;
-    p->bp_bulk = g->storage == AT3R_STORE_F32 && (g->nx & 3) == 0 && bp_bulk_from_env() ? 1 : 0;
     p->N = g->nx & ~1; p->Nx = p->N; p->Nz = g->vol_z; p->KX = p->Nx / 2 + 1;
     cudaGetDevice(&p->device);
 
@@ -805,10 +783,9 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
         for (int i = 1; i < k; i++) p->sub_start[i] = p->sub_start[i - 1] + p->sub_size[i - 1];
         p->bp_ww_sart = bp_window(BP_TX, BP_TZ, 1.0, cs, p->T);
         if (p->bp_ww_sart > BP_WW) return fail(set_err(AT3R_ERR_TOO_LARGE, "back-projection window exceeds its stride"));
-        for (const void* fn : {(const void*)k_bp<0, float, float, true>, (const void*)k_bp<0, __half, __half, true>,
-                               (const void*)k_bp<0, __nv_bfloat16, __nv_bfloat16, true>})
-            if ((rc = set_smem(fn, bp_smem(0)))) return fail(rc);
-        if (p->bp_bulk && (rc = set_smem((const void*)k_bp<0, float, float, true, true>, bp_smem(1)))) return fail(rc);
+        for (const void* fn : {(const void*)k_bp<float, float, true>, (const void*)k_bp<__half, __half, true>,
+                               (const void*)k_bp<__nv_bfloat16, __nv_bfloat16, true>})
+            if ((rc = set_smem(fn, bp_smem_bytes()))) return fail(rc);
         if (p->wide) {
             for (auto& f : {std::make_pair((const void*)k_fp_wide<64>, Fpw<64>::SMEM),
                             std::make_pair((const void*)k_fp_wide<32>, Fpw<32>::SMEM),
@@ -853,8 +830,6 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
         p->zcrop_cb = std::max(4, std::min(32, 4096 / (2 * p->Nz)));
         while (p->zcrop_cb > 1 && 2 * sizeof(float2) * p->zcrop_cb * p->zcrop_pitch > 227 * 1024) p->zcrop_cb /= 2;
         p->smem_zcrop = 2 * sizeof(float2) * p->zcrop_cb * p->zcrop_pitch;
-        p->bp_ww_wbp = bp_window(BP_TX, BP_TZ, 0.5, cs, p->T);
-        if (p->bp_ww_wbp > BP_WW) return fail(set_err(AT3R_ERR_TOO_LARGE, "back-projection window exceeds its stride"));
         p->rs_zcrop = std::max(p->f2z.rs, p->fz.rs);
         std::vector<std::pair<const void*, size_t>> fns;
         dispatch_rs(p->fN.rs, [&](auto R) {
@@ -868,10 +843,6 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
         dispatch_rs(p->fx.rs, [&](auto R) { fns.push_back({(const void*)k_x_c2r<decltype(R)::value>, p->smem_xc2r}); });
         for (auto& f : fns)
             if ((rc = set_smem(f.first, f.second))) return fail(rc);
-        for (const void* fn : {(const void*)k_bp<1, float, float, false>, (const void*)k_bp<1, __half, float, false>,
-                               (const void*)k_bp<1, __nv_bfloat16, float, false>})
-            if ((rc = set_smem(fn, bp_smem(0)))) return fail(rc);
-        if (p->bp_bulk && (rc = set_smem((const void*)k_bp<1, float, float, false, true>, bp_smem(1)))) return fail(rc);
         // R-weight transfer function (GRWeight.cu:15-20), 1/N folded in
         std::vector<float> h(N / 2 + 1);
         const double twopi = (double)6.2831852f;
@@ -1529,7 +1500,7 @@ at3r_status noalloc_scratch_address(unsigned char** out)
         return set_err(AT3R_ERR_CUDA, std::string("cudaGetSymbolAddress(no-allocation scratch): ") +
                                           cudaGetErrorString(e));
     }
-    at3r_status rc = set_smem((const void*)k_bp<0, float, float, false>, 0);
+    at3r_status rc = set_smem((const void*)k_bp<float, float, false>, 0);
     if (rc != AT3R_OK) return rc;
     *out = (unsigned char*)ptr;
     return AT3R_OK;
@@ -1582,7 +1553,7 @@ extern "C" at3r_status at3r_sart_device_noalloc(const float* proj, int nx, int n
     }
     const int ww = bp_window(BP_TX, BP_TZ, 1.0, cs, T);
     if (ww > BP_WW) return set_err(AT3R_ERR_TOO_LARGE, "back-projection window exceeds its stride");
-    if (bp_smem(0) > 227 * 1024) return set_err(AT3R_ERR_TOO_LARGE, "back-projection window exceeds 227 KB");
+    if (bp_smem_bytes() > 227 * 1024) return set_err(AT3R_ERR_TOO_LARGE, "back-projection window exceeds 227 KB");
     unsigned char* base = nullptr;
     at3r_status rc = noalloc_scratch_address(&base);
     if (rc != AT3R_OK) return rc;
@@ -1623,7 +1594,7 @@ extern "C" at3r_status at3r_sart_device_noalloc(const float* proj, int nx, int n
         a.out = v; a.out_slice = (size_t)Nx * Nz; a.ww = ww; a.flags = d_flags;
         const dim3 bgrid((Nx + BP_TX - 1) / BP_TX, (Nz + BP_TZ - 1) / BP_TZ, SG);
         a.sino = d_raw; a.t0 = 0; a.t1 = T; a.relax = 1.f; a.low_bit = kFlagRawLow;
-        k_bp<0, float, float, false><<<bgrid, BP_THREADS, bp_smem(0), st>>>(a);
+        k_bp<float, float, false><<<bgrid, BP_THREADS, bp_smem_bytes(), st>>>(a);
         AT3R_CUDA(cudaGetLastError());
         a.sino = d_diff; a.relax = rlx; a.low_bit = kFlagDiffLow;
         for (int it = 0; it < iterations; it++) {
@@ -1635,7 +1606,7 @@ extern "C" at3r_status at3r_sart_device_noalloc(const float* proj, int nx, int n
                                                                                        d_flags);
                 AT3R_CUDA(cudaGetLastError());
                 a.t0 = t0; a.t1 = t0 + nt;
-                k_bp<0, float, float, false><<<bgrid, BP_THREADS, bp_smem(0), st>>>(a);
+                k_bp<float, float, false><<<bgrid, BP_THREADS, bp_smem_bytes(), st>>>(a);
                 AT3R_CUDA(cudaGetLastError());
             }
         }
@@ -1761,16 +1732,12 @@ at3r_status build_waves(at3r_batch* b)
             d.zcrop_cb = p->zcrop_cb; d.zcrop_pitch = p->zcrop_pitch;
             d.packed = p->c2r == AT3R_C2R_PACKED;
             d.norm = (float)(1.0 / (2.0 * Nx) / (2.0 * Nz));
-            BpArgs& a = d.bp;
-            a.sino = filt; a.scale = scale; a.shadow = nullptr; a.T = T; a.N = N; a.t0 = 0; a.t1 = T;
-            a.cs = p->d_cs; a.GX = 2 * Nx; a.GZ = 2 * Nz; a.S = S; a.relax = 1.f; a.out = g2;
-            a.out_slice = (size_t)4 * Nx * Nz; a.ww = p->bp_ww_wbp; a.flags = flags; a.seen = p->d_seen;
-            a.low_bit = kFlagRawLow; a.bulk = 0;
+            d.bp = wbp_args(p, S, filt, scale, flags, g2);
             d.fN = p->fN.plan; d.f2x = p->f2x.plan; d.f2z = p->f2z.plan; d.fz = p->fz.plan; d.fx = p->fx.plan;
             d.gx[0] = ((T + 1) / 2 + p->b_rweight - 1) / p->b_rweight;
-            d.gx[1] = (2 * Nx + BP_TX - 1) / BP_TX;
-            d.bp_gy = (2 * Nz + BP_TZ - 1) / BP_TZ;
-            d.bp_gz = (S + SB - 1) / SB;
+            d.gx[1] = (2 * Nx + WBP_T - 1) / WBP_T;
+            d.bp_gy = (2 * Nz + WBP_T - 1) / WBP_T;
+            d.bp_gz = (S + WBP_WAVE_SLICES - 1) / WBP_WAVE_SLICES;
             d.gx[2] = (Nz + p->b_row - 1) / p->b_row;
             d.gx[3] = (KX + p->zcrop_cb - 1) / p->zcrop_cb;
             d.gx[4] = ((Nz + 1) / 2 + p->b_xc2r - 1) / p->b_xc2r;
@@ -1806,7 +1773,7 @@ at3r_status build_waves(at3r_batch* b)
         b->smem[3] = std::max(b->smem[3], p->smem_zcrop);
         b->smem[4] = std::max(b->smem[4], p->smem_xc2r);
     }
-    b->smem[1] = bp_smem(0);
+    b->smem[1] = wbp_bp_smem<WBP_WAVE_SLICES>();
     const void* fn[kWbpStages];
     wave_kernels_of(b->storage, b->rs, fn);
     int dev = 0, sms = 148;
@@ -1816,7 +1783,7 @@ at3r_status build_waves(at3r_batch* b)
         at3r_status rc = set_smem(fn[k], b->smem[k]);
         if (rc) return rc;
         int per_sm = 0;
-        AT3R_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn[k], k == 1 ? BP_THREADS : 512, b->smem[k]));
+        AT3R_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn[k], k == 1 ? WBP_THREADS : 512, b->smem[k]));
         b->grid[k] = std::max(1, per_sm) * sms;
     }
     b->waves = true;
@@ -1846,7 +1813,7 @@ at3r_status run_waves(at3r_batch* b, cudaStream_t st0, cudaStream_t st1, cudaEve
             int* counter = b->d_counters + w * kWbpStages + k;
             int nslabs = nw;
             void* args[] = {(void*)&ds, (void*)&start, (void*)&nslabs, (void*)&counter};
-            AT3R_CUDA(cudaLaunchKernel(fn[k], dim3(b->grid[k]), dim3(k == 1 ? BP_THREADS : 512), args, b->smem[k], st));
+            AT3R_CUDA(cudaLaunchKernel(fn[k], dim3(b->grid[k]), dim3(k == 1 ? WBP_THREADS : 512), args, b->smem[k], st));
         }
     }
     return AT3R_OK;

@@ -169,6 +169,7 @@ constexpr int kFlagRawLow = 2;      // the staged sinogram holds values <= kLowV
 constexpr int kFlagDiffLow = 4;     // the residual holds values <= kLowValue
 constexpr int kFlagRawSpecial = 32, kFlagDiffSpecial = 64, kFlagVolSpecial = 128;   // see sart_wide.cuh
 constexpr int kFlagsReported = 31;  // the bits of the run summary
+constexpr float kSpecial = 1e30f;   // values beyond it, infinities and NaN: kFlag*Special
 constexpr float kLowValue = -5.0e9f;  // far from any lerp of values above it reaching -1e10
 
 // y-slices one thread carries: every slice has the same geometry (single
@@ -281,7 +282,7 @@ __device__ __forceinline__ void rweight_block(const float* __restrict__ proj, si
         }
         __syncthreads();
     }
-    bool low = false;
+    bool low = false, special = false;
     for (int q = 0; q < nq; q++) {
         const int t0 = 2 * (pair0 + q);
         const bool two = t0 + 1 < T;
@@ -293,13 +294,15 @@ __device__ __forceinline__ void rweight_block(const float* __restrict__ proj, si
             const float2 v = rq[fft_pad(x)];
             Stor<ST>::st(d0 + x, v.x, inv0);
             low |= v.x <= kLowValue;
+            special |= !(fabsf(v.x) < kSpecial);
             if (two) {
                 Stor<ST>::st(d0 + N + x, v.y, inv1);
                 low |= v.y <= kLowValue;
+                special |= !(fabsf(v.y) < kSpecial);
             }
         }
     }
-    if (low) atomicOr(flags + ys, kFlagRawLow);
+    if (low || special) atomicOr(flags + ys, (low ? kFlagRawLow : 0) | (special ? kFlagRawSpecial : 0));
 }
 
 template <typename ST, int RS>
@@ -313,11 +316,10 @@ __global__ void __launch_bounds__(512, RS < 2 ? 2 : 1) k_rweight(const float* __
 }
 
 // ---------------------------------------------------------------------------
-// Back-projection.  MODE 0: SART update on the 1x grid
+// Back-projection: SART update on the 1x grid, series of a few rows and the
+// no-allocation entry point (sart_wide.cuh has the others, wbp_bp.cuh the WBP grid)
 // (AreTomo/Recon/GBackProj.cu:12-60, bSart): the mean over tilts [t0, t1) of
-// the lerped sinogram is scaled by relax, added, clamped at 0.  MODE 1: the
-// WBP 2x grid (AreTomo/Recon/GBackProjWbp.cu:14-53): mean over all tilts,
-// or 0 where no tilt contributes.
+// the lerped sinogram is scaled by relax, added, clamped at 0.
 //
 // A CTA covers BP_TX x BP_TZ voxels of SB slices; each thread keeps 2 x 4
 // voxel positions (x warp-contiguous) for all SB slices.  Tilts go in chunks
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(512, RS < 2 ? 2 : 1) k_rweight(const float* __
 constexpr int BP_TX = 64, BP_TZ = 32, BP_THREADS = 256, BP_CHUNK = 16;
 // Shared-memory stride of one tilt's staged window (pairs).  A window spans
 // at most |cos|(BP_TX - 1) + |sin|(BP_TZ - 1) + 6 <= sqrt(63^2 + 31^2) + 6 < 77
-// samples (cos^2 + sin^2 = 1; the WBP grid halves it), so a fixed stride
+// samples (cos^2 + sin^2 = 1), so a fixed stride
 // holds every case and makes the per-slice offsets immediates.
 constexpr int BP_WW = 80;
 constexpr int BP_PSLAB = BP_CHUNK * BP_WW;   // pairs per slice
@@ -346,21 +348,21 @@ struct BpArgs {
     const float* scale;      // [slices][T] row scales (16-bit storage), else null
     int T, N, t0, t1;
     const float2* cs;
-    int GX, GZ;              // voxel grid of this mode
+    int GX, GZ;              // voxel grid
     int S;                   // slices in this launch
     float relax;
-    float* out;              // MODE 0: vol slab [slices][GZ][GX] (z flipped), or the slice-group volume
-                             // [groups][GZ][GX] float4; MODE 1: [slices][GZ][GX]
+    float* out;              // vol slab [slices][GZ][GX] (z flipped), or the slice-group volume
+                             // [groups][GZ][GX] float4
     size_t out_slice;
     int ww;                  // staged window width (samples)
     int* flags;              // per-slice flag bits
     int low_bit;             // the flag bit that marks this sinogram as holding low values
-    void* shadow;            // MODE 0, 16-bit volume type: [ceil(slices/8)][GZ][GX] of eight 16-bit values
+    void* shadow;            // 16-bit volume type: [ceil(slices/8)][GZ][GX] of eight 16-bit values
                              // beside the slice-group volume (shadow_half)
     int* seen;               // run summary: the flags of every slice ORed in (may be null)
-    int bulk;                // FP32 storage, N % 4 == 0: launch the bulk-copy staging form (bp_smem_bytes(1))
 };
 
+// Detector position of a voxel.  MODE 0: the SART grid; 1: the WBP 2x grid.
 template <int MODE>
 __device__ __forceinline__ float bp_xp(float fX, float fZs, float c, float cent)
 {
@@ -372,15 +374,22 @@ __device__ __forceinline__ float bp_xp(float fX, float fZs, float c, float cent)
     return __fadd_rn(__fmaf_rn(a, 0.5f, cent), 0.5f);
 }
 
-// Raw window rows of the bulk-copy staging: a row is copied from the 16-byte
-// boundary at or below its window start, so it spans at most 3 + 81 floats.
-constexpr int BP_RAW_W = 88;
-constexpr int kFlagStageTimeout = 16;   // a bulk staging wait ran out (the tile was not written)
+constexpr int kFlagStageTimeout = 16;   // a bulk copy did not arrive (the output was not written)
 
-__host__ __device__ inline size_t bp_smem_bytes(int bulk)
+__host__ __device__ inline size_t bp_smem_bytes()
 {
-    const size_t base = (sizeof(int) + sizeof(float2)) * BP_CHUNK + sizeof(float2) * (size_t)SB * BP_PSLAB;
-    return bulk ? base + 16 + sizeof(float) * (size_t)SB * BP_CHUNK * BP_RAW_W : base;
+    return (sizeof(int) + sizeof(float2)) * BP_CHUNK + sizeof(float2) * (size_t)SB * BP_PSLAB;
+}
+
+// Two FP32 fused multiply-adds in one instruction (the same rate per
+// multiply-add as the scalar form, half the issue slots).
+__device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b)
+{
+    unsigned long long r = *reinterpret_cast<unsigned long long*>(&acc);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;"
+        : "+l"(r)
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    acc = *reinterpret_cast<float2*>(&r);
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -401,31 +410,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int lim
     return false;
 }
 
-// Writes one voxel and returns its value afterwards (the old value where no
-// tilt contributed).
-// k: relax / cnt (MODE 0) or 1 / cnt (MODE 1), one division per voxel for
+// Updates one voxel of the plain volume; k: relax / cnt, one division per voxel for
 // all its slices.
-template <int MODE>
-__device__ __forceinline__ float bp_store(const BpArgs& p, int ys, int Z, int X, float sum, int cnt, float k)
+__device__ __forceinline__ void bp_store(const BpArgs& p, int ys, int Z, int X, float sum, int cnt, float k)
 {
-    float* out = p.out + (size_t)ys * p.out_slice;
-    if (MODE == 0) {
-        float* v = out + (size_t)(p.GZ - 1 - Z) * p.GX + X;
-        if (cnt <= 0) return *v;
-        const float f = __fadd_rn(__fmul_rn(sum, k), *v);
-        if (f > kSentinelTest) {
-            const float r = fmaxf(f, 0.f);
-            *v = r;
-            return r;
-        }
-        *v = kSentinelValue;
-        atomicOr(p.flags + ys, kFlagVolEmpty);
-        return kSentinelValue;
-    } else {
-        const float r = cnt > 0 ? __fmul_rn(sum, k) : 0.f;
-        out[(size_t)Z * p.GX + X] = r;
-        return r;
+    if (cnt <= 0) return;
+    float* v = p.out + (size_t)ys * p.out_slice + (size_t)(p.GZ - 1 - Z) * p.GX + X;
+    const float f = __fadd_rn(__fmul_rn(sum, k), *v);
+    if (f > kSentinelTest) {
+        *v = fmaxf(f, 0.f);
+        return;
     }
+    *v = kSentinelValue;
+    atomicOr(p.flags + ys, kFlagVolEmpty);
 }
 
 // The 16-bit shadow of the SART working volume holds eight slices per voxel
@@ -493,41 +490,20 @@ __device__ __forceinline__ void bp_store1_grp(const BpArgs& p, int g, int q, int
         Quad<VT>::st1(reinterpret_cast<uint2*>(p.shadow) + shadow_half(p, g, Z, X), q, r);
 }
 
-// GRP (MODE 0 only): the volume is the slice-group working volume above;
-// otherwise MODE 0 updates a plain [slices][GZ][GX] volume (z flipped).
-// BULK (FP32 storage, N a multiple of 4): window rows staged by bulk
-// asynchronous copies, the comparison form; the default form has none of its code.
-template <int MODE, typename ST, typename VT, bool GRP, bool BULK = false>
+// GRP: the volume is the slice-group working volume above; otherwise a plain
+// [slices][GZ][GX] volume (z flipped).
+template <typename ST, typename VT, bool GRP>
 __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
 {
-    // FP16 WBP (MODE 1) stages FP16 values and differences (below); SART keeps
-    // the FP32 pairs, where the per-sample conversion of the fraction to FP16
-    // cost more than the halved shared-memory bytes saved
-    constexpr bool H2 = std::is_same<ST, __half>::value && MODE == 1;
-    static_assert(!GRP || MODE == 0, "the slice-group layout is the SART working volume");
     static_assert(GRP || std::is_same<VT, float>::value, "the 16-bit shadow exists in the slice-group layout only");
     extern __shared__ float2 bsm[];
     float2* cs_s = bsm;                                               // [BP_CHUNK]
     float2* pw = bsm + BP_CHUNK;                                      // [SB][BP_CHUNK][BP_WW]
     int* ws = reinterpret_cast<int*>(pw + SB * BP_PSLAB);             // [BP_CHUNK]
-    // bulk staging: an mbarrier and the raw rows [SB][BP_CHUNK][BP_RAW_W]
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(ws + BP_CHUNK);
-    float* raw = reinterpret_cast<float*>(reinterpret_cast<char*>(mbar) + 16);
-    constexpr bool bulk = BULK && std::is_same<ST, float>::value;
-    uint32_t phase = 0;
-    bool stage_ok = true;
-    if (bulk) {
-        if (threadIdx.x == 0) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        __syncthreads();
-    }
     const int ys0 = bz * SB, nsl = min(SB, p.S - ys0);
     const int X0 = bx * BP_TX, Z0 = by * BP_TZ;
-    const float cent = MODE == 0 ? (float)p.N / 2.0f : (float)(p.N / 2);
-    const float hx = MODE == 0 ? (float)p.GX * 0.5f : (float)p.GX / 2.0f;
-    const float hz = MODE == 0 ? (float)p.GZ * 0.5f : (float)p.GZ / 2.0f;
+    const float cent = (float)p.N / 2.0f;
+    const float hx = (float)p.GX * 0.5f, hz = (float)p.GZ * 0.5f;
     const float endX = (float)(p.N - 2);
     const unsigned wmax = (unsigned)(p.ww - 2);
 
@@ -537,28 +513,6 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
         atomicOr(p.seen, __ldg(p.flags + ys0 + threadIdx.x));
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // H2: the fast path stages each window position as FP16 values and
-    // differences in a common scale per slice (2^-12 of the largest row scale
-    // of the launch's tilts), so a sample interpolates two slices per fma.f16x2
-    __shared__ float ssc[SB];
-    __shared__ float rq[SB][BP_CHUNK];
-    float slice_scale[SB];
-    if constexpr (H2) {
-        if (warp < SB) {
-            float m = 0.f;
-            if (warp < nsl)
-                for (int t = p.t0 + lane; t < p.t1; t += 32) m = fmaxf(m, __ldg(p.scale + (size_t)(ys0 + warp) * p.T + t));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            // 2^-12 of the largest row scale: the largest values stage as up to
-            // 4096 (FP16 holds 65504), and rows far weaker than the strongest
-            // stay above FP16's subnormal range
-            if (lane == 0) ssc[warp] = m > 0.f ? m * 0x1p-12f : 1.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < SB; q++) slice_scale[q] = ssc[q];
-    }
     float fX[BP_CX], fZ[BP_CZ];
 #pragma unroll
     for (int i = 0; i < BP_CX; i++) fX[i] = (float)(X0 + lane + 32 * i) - hx;
@@ -567,14 +521,8 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
 
     // stage chunk [c0, c0 + nc) of slices [ys0, ys0 + ns) into pw; returns
     // whether the whole tile stays strictly inside the detector for it
-    auto stage = [&](int c0, int nc, int ysA, int ns, bool h2) -> bool {
+    auto stage = [&](int c0, int nc, int ysA, int ns) -> bool {
         int inside = 1;
-        if (H2 && h2 && threadIdx.x < nc) {
-#pragma unroll
-            for (int q = 0; q < SB; q++)
-                rq[q][threadIdx.x] =
-                    q < ns ? __fdiv_rn(__ldg(p.scale + (size_t)(ysA + q) * p.T + c0 + threadIdx.x), ssc[q]) : 0.f;
-        }
         if (threadIdx.x < nc) {
             const float2 c = __ldg(&p.cs[c0 + threadIdx.x]);
             float lo = 3.0e38f, hi = -3.0e38f;
@@ -582,7 +530,7 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
             for (int k = 0; k < 4; k++) {
                 const float cX = (float)(X0 + ((k & 1) ? BP_TX - 1 : 0)) - hx;
                 const float cZ = (float)(Z0 + ((k & 2) ? BP_TZ - 1 : 0)) - hz;
-                const float xp = bp_xp<MODE>(cX, __fmul_rn(cZ, c.y), c.x, cent);
+                const float xp = bp_xp<0>(cX, __fmul_rn(cZ, c.y), c.x, cent);
                 lo = fminf(lo, xp);
                 hi = fmaxf(hi, xp);
             }
@@ -591,82 +539,6 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
             inside = (lo >= 0.01f) && (hi <= endX - 0.01f);
         }
         inside = __syncthreads_and(inside);
-        if constexpr (H2) {
-            if (h2) {
-                // entry (t, k) = {v0 v1, v2 v3, d0 d1, d2 d3} (FP16): v_q the value of
-                // slice q at window position k, d_q = v_q(k + 1) - v_q(k), both in
-                // units of the slice's scale; slices past the slab stay zero.  One
-                // warp per tilt, lanes along the window.  (No value here is a
-                // missing-value marker: a row holding one flags its slice, which
-                // takes the per-slice path.)
-                uint4* ph = reinterpret_cast<uint4*>(pw);
-                constexpr int NW = BP_THREADS / 32;
-                for (int t = warp; t < nc; t += NW) {
-                    const int x0 = ws[t];
-                    const bool on = x0 >= 0 && x0 + p.ww + 1 <= p.N;   // warp-uniform
-                    for (int k = lane; k < p.ww; k += 32) {
-                        const int x = x0 + k;
-                        float v[SB], d[SB];
-#pragma unroll
-                        for (int q = 0; q < SB; q++) {
-                            float a = 0.f, b = 0.f;
-                            if (q < ns) {
-                                const __half* src =
-                                    reinterpret_cast<const __half*>(p.sino) + ((size_t)(ysA + q) * p.T + c0 + t) * p.N;
-                                if (on || (x >= 0 && x < p.N)) a = __half2float(__ldg(src + x));
-                                if (on || (x + 1 >= 0 && x + 1 < p.N)) b = __half2float(__ldg(src + x + 1));
-                            }
-                            const float r = rq[q][t];
-                            v[q] = __fmul_rn(a, r);
-                            d[q] = __fmul_rn(__fsub_rn(b, a), r);
-                        }
-                        ph[t * BP_WW + k] = make_uint4(bits_of(__floats2half2_rn(v[0], v[1])),
-                                                       bits_of(__floats2half2_rn(v[2], v[3])),
-                                                       bits_of(__floats2half2_rn(d[0], d[1])),
-                                                       bits_of(__floats2half2_rn(d[2], d[3])));
-                    }
-                }
-                __syncthreads();
-                return inside != 0;
-            }
-        }
-        // bulk staging (FP32): a row whose copy range — from the 16-byte boundary
-        // at or below its window start through the window's last sample, rounded
-        // up to 16 bytes — lies on the detector is fetched by one bulk
-        // asynchronous copy (warp 0, one row per lane, completion counted by
-        // the mbarrier); other rows take the load path below
-        auto bulk_row = [&](int t, int& xa, int& nf) {
-            const int x0 = ws[t];
-            xa = x0 & ~3;
-            nf = (x0 + p.ww + 1 - xa + 3) & ~3;
-            return xa >= 0 && xa + nf <= p.N;
-        };
-        if (bulk && warp == 0) {
-            uint32_t bytes = 0;
-            for (int r = lane; r < ns * nc; r += 32) {
-                int xa, nf;
-                if (bulk_row(r % nc, xa, nf)) bytes += 4u * nf;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
-            if (lane == 0) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes)
-                             : "memory");
-            }
-            __syncwarp();
-            for (int r = lane; r < ns * nc; r += 32) {
-                const int q = r / nc, t = r - q * nc;
-                int xa, nf;
-                if (!bulk_row(t, xa, nf)) continue;
-                const float* src = reinterpret_cast<const float*>(p.sino) + ((size_t)(ysA + q) * p.T + c0 + t) * p.N + xa;
-                asm volatile(
-                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                        smem_u32(raw + (q * BP_CHUNK + t) * BP_RAW_W)),
-                    "l"(src), "r"(4u * nf), "r"(smem_u32(mbar))
-                    : "memory");
-            }
-        }
         // one warp per (slice, tilt) row, lanes along the window; a lane issues
         // all its loads of the row before its first store, so a warp waits for
         // the L2 once per row rather than once per load
@@ -676,14 +548,6 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
         int q = warp / nc, t = warp - (warp / nc) * nc;
         for (int row = warp; row < ns * nc; row += NW) {
             const int x0 = ws[t];
-            if (bulk) {
-                int xa, nf;
-                if (bulk_row(t, xa, nf)) {
-                    t += NW;
-                    while (t >= nc) { t -= nc; q++; }
-                    continue;
-                }
-            }
             const size_t row_id = (size_t)(ysA + q) * p.T + c0 + t;
             const float sc = std::is_same<ST, float>::value ? 1.f : __ldg(p.scale + row_id);
             const ST* src = reinterpret_cast<const ST*>(p.sino) + row_id * p.N + x0 + lane;
@@ -712,34 +576,12 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
             t += NW;
             while (t >= nc) { t -= nc; q++; }
         }
-        if (bulk) {
-            // every thread waits for the copies (a bounded wait: on timeout the
-            // tile is flagged and left unwritten), then the raw rows become pairs
-            const bool ok = mbar_wait(smem_u32(mbar), phase, 1 << 22);
-            stage_ok = __syncthreads_and(ok && stage_ok) != 0;
-            if (stage_ok) phase ^= 1;
-            for (int e = threadIdx.x; stage_ok && e < ns * nc * p.ww; e += BP_THREADS) {
-                const int r = e / p.ww, k = e - r * p.ww;
-                const int q = r / nc, t = r - q * nc;
-                int xa, nf;
-                if (!bulk_row(t, xa, nf)) continue;
-                const float* rr = raw + (q * BP_CHUNK + t) * BP_RAW_W + (ws[t] - xa) + k;
-                pw[q * BP_PSLAB + t * BP_WW + k] = make_float2(rr[0], rr[1]);
-            }
-        }
         __syncthreads();
         return inside != 0;
     };
 
-    // a bulk staging wait that ran out: wait once more (bounded) for the
-    // copies still in flight, flag the slab, write nothing
-    auto give_up = [&]() {
-        mbar_wait(smem_u32(mbar), phase, 1 << 22);
-        if (threadIdx.x == 0) atomicOr(p.flags + ys0, kFlagStageTimeout);
-    };
-
     if (!low) {
-        if (!H2 && GRP && nsl < SB) {
+        if (GRP && nsl < SB) {
             // rows of slices past the slab's end stay zero (staging never writes them)
             for (int k = threadIdx.x; k < (SB - nsl) * BP_PSLAB; k += BP_THREADS)
                 pw[nsl * BP_PSLAB + k] = make_float2(0.f, 0.f);
@@ -756,66 +598,8 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
             }
         for (int c0 = p.t0; c0 < p.t1; c0 += BP_CHUNK) {
             const int nc = min(BP_CHUNK, p.t1 - c0);
-            const bool inside = stage(c0, nc, ys0, nsl, true);
-            if (!stage_ok) break;
-            if (H2 && inside) {
-                const uint4* ph = reinterpret_cast<const uint4*>(pw);
-                for (int t = 0; t < nc; t++) {
-                    const float2 c = cs_s[t];
-                    const int wb = t * BP_WW - ws[t] - kMagicBits;
-#pragma unroll
-                    for (int j = 0; j < BP_CZ; j++) {
-                        const float fzs = __fmul_rn(fZ[j], c.y);
-#pragma unroll
-                        for (int i = 0; i < BP_CX; i++) {
-                            const float xp = bp_xp<MODE>(fX[i], fzs, c.x, cent);
-                            const float tr = __fadd_rd(xp, kMagic);
-                            const float fr = __fsub_rn(xp, __fsub_rn(tr, kMagic));
-                            const uint4 e = ph[__float_as_int(tr) + wb];
-                            const __half2 f2 = __float2half2_rn(fr);
-                            const __half2 v01 = __hfma2(from_bits<__half2>(e.z), f2, from_bits<__half2>(e.x));
-                            const __half2 v23 = __hfma2(from_bits<__half2>(e.w), f2, from_bits<__half2>(e.y));
-                            sum[0][j][i] = add_f32_f16(sum[0][j][i], __low2half(v01));
-                            sum[1][j][i] = add_f32_f16(sum[1][j][i], __high2half(v01));
-                            sum[2][j][i] = add_f32_f16(sum[2][j][i], __low2half(v23));
-                            sum[3][j][i] = add_f32_f16(sum[3][j][i], __high2half(v23));
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < BP_CZ; j++)
-#pragma unroll
-                    for (int i = 0; i < BP_CX; i++) cnt[j][i] += nc;
-            } else if (H2) {
-                const uint4* ph = reinterpret_cast<const uint4*>(pw);
-                for (int t = 0; t < nc; t++) {
-                    const float2 c = cs_s[t];
-                    const uint4* w = ph + t * BP_WW;
-                    const int st = ws[t];
-#pragma unroll
-                    for (int j = 0; j < BP_CZ; j++) {
-                        const float fzs = __fmul_rn(fZ[j], c.y);
-#pragma unroll
-                        for (int i = 0; i < BP_CX; i++) {
-                            const float xp = bp_xp<MODE>(fX[i], fzs, c.x, cent);
-                            const bool in = xp >= 0.f && xp <= endX;
-                            const int ii = (int)xp;
-                            const float fr = __fsub_rn(xp, (float)ii);
-                            const uint4 e = w[min((unsigned)(ii - st), wmax)];
-                            const __half2 f2 = __float2half2_rn(fr);
-                            const __half2 v01 = __hfma2(from_bits<__half2>(e.z), f2, from_bits<__half2>(e.x));
-                            const __half2 v23 = __hfma2(from_bits<__half2>(e.w), f2, from_bits<__half2>(e.y));
-                            if (in) {
-                                sum[0][j][i] = add_f32_f16(sum[0][j][i], __low2half(v01));
-                                sum[1][j][i] = add_f32_f16(sum[1][j][i], __high2half(v01));
-                                sum[2][j][i] = add_f32_f16(sum[2][j][i], __low2half(v23));
-                                sum[3][j][i] = add_f32_f16(sum[3][j][i], __high2half(v23));
-                                cnt[j][i] += 1;
-                            }
-                        }
-                    }
-                }
-            } else if (inside) {
+            const bool inside = stage(c0, nc, ys0, nsl);
+            if (inside) {
                 // the whole tile lands inside the detector for every tilt of the chunk
                 for (int t = 0; t < nc; t++) {
                     const float2 c = cs_s[t];
@@ -826,7 +610,7 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
                         const float fzs = __fmul_rn(fZ[j], c.y);
 #pragma unroll
                         for (int i = 0; i < BP_CX; i++) {
-                            const float xp = bp_xp<MODE>(fX[i], fzs, c.x, cent);
+                            const float xp = bp_xp<0>(fX[i], fzs, c.x, cent);
                             const float tr = __fadd_rd(xp, kMagic);
                             const float fr = __fsub_rn(xp, __fsub_rn(tr, kMagic));
                             const float om = __fsub_rn(1.f, fr);
@@ -853,7 +637,7 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
                         const float fzs = __fmul_rn(fZ[j], c.y);
 #pragma unroll
                         for (int i = 0; i < BP_CX; i++) {
-                            const float xp = bp_xp<MODE>(fX[i], fzs, c.x, cent);
+                            const float xp = bp_xp<0>(fX[i], fzs, c.x, cent);
                             const bool in = xp >= 0.f && xp <= endX;
                             const int ii = (int)xp;
                             const float fr = __fsub_rn(xp, (float)ii);
@@ -872,10 +656,6 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
             }
             __syncthreads();
         }
-        if (!stage_ok) {
-            give_up();
-            return;
-        }
 #pragma unroll
         for (int j = 0; j < BP_CZ; j++) {
             const int Z = Z0 + warp + (BP_THREADS / 32) * j;
@@ -883,18 +663,14 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
             for (int i = 0; i < BP_CX; i++) {
                 const int X = X0 + lane + 32 * i;
                 if (Z >= p.GZ || X >= p.GX) continue;
-                if constexpr (H2) {
-#pragma unroll
-                    for (int q = 0; q < SB; q++) sum[q][j][i] = __fmul_rn(sum[q][j][i], slice_scale[q]);
-                }
                 if constexpr (GRP) {
                     bp_store_grp<VT>(p, bz, ys0, nsl, Z, X,
                                      make_float4(sum[0][j][i], sum[1][j][i], sum[2][j][i], sum[3][j][i]), cnt[j][i]);
                 } else {
-                    const float k = cnt[j][i] > 0 ? __fdiv_rn(MODE == 0 ? p.relax : 1.f, (float)cnt[j][i]) : 0.f;
+                    const float k = cnt[j][i] > 0 ? __fdiv_rn(p.relax, (float)cnt[j][i]) : 0.f;
 #pragma unroll
                     for (int q = 0; q < SB; q++)
-                        if (q < nsl) bp_store<MODE>(p, ys0 + q, Z, X, sum[q][j][i], cnt[j][i], k);
+                        if (q < nsl) bp_store(p, ys0 + q, Z, X, sum[q][j][i], cnt[j][i], k);
                 }
             }
         }
@@ -911,8 +687,7 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
             for (int i = 0; i < BP_CX; i++) { sum[j][i] = 0.f; cnt[j][i] = 0; }
         for (int c0 = p.t0; c0 < p.t1; c0 += BP_CHUNK) {
             const int nc = min(BP_CHUNK, p.t1 - c0);
-            stage(c0, nc, ys0 + q, 1, false);
-            if (!stage_ok) break;
+            stage(c0, nc, ys0 + q, 1);
             for (int t = 0; t < nc; t++) {
                 const float2 c = cs_s[t];
                 const float2* w = pw + t * BP_WW;
@@ -922,7 +697,7 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
                     const float fzs = __fmul_rn(fZ[j], c.y);
 #pragma unroll
                     for (int i = 0; i < BP_CX; i++) {
-                        const float xp = bp_xp<MODE>(fX[i], fzs, c.x, cent);
+                        const float xp = bp_xp<0>(fX[i], fzs, c.x, cent);
                         const int ii = (int)xp;
                         const float fr = __fsub_rn(xp, (float)ii);
                         const float2 v2 = w[min((unsigned)(ii - st), wmax)];
@@ -937,10 +712,6 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
             }
             __syncthreads();
         }
-        if (!stage_ok) {
-            give_up();
-            return;
-        }
 #pragma unroll
         for (int j = 0; j < BP_CZ; j++) {
             const int Z = Z0 + warp + (BP_THREADS / 32) * j;
@@ -951,8 +722,8 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
                     if constexpr (GRP) {
                         bp_store1_grp<VT>(p, bz, q, ys0 + q, Z, X, sum[j][i], cnt[j][i]);
                     } else {
-                        const float k = cnt[j][i] > 0 ? __fdiv_rn(MODE == 0 ? p.relax : 1.f, (float)cnt[j][i]) : 0.f;
-                        bp_store<MODE>(p, ys0 + q, Z, X, sum[j][i], cnt[j][i], k);
+                        const float k = cnt[j][i] > 0 ? __fdiv_rn(p.relax, (float)cnt[j][i]) : 0.f;
+                        bp_store(p, ys0 + q, Z, X, sum[j][i], cnt[j][i], k);
                     }
                 }
             }
@@ -968,15 +739,15 @@ __device__ __forceinline__ void bp_tile(BpArgs p, int bx, int by, int bz)
 template <typename VT>
 __host__ __device__ constexpr bool bp_paired() { return !std::is_same<VT, float>::value; }
 
-template <int MODE, typename ST, typename VT, bool GRP, bool BULK = false>
+template <typename ST, typename VT, bool GRP>
 __global__ void __launch_bounds__(BP_THREADS, 3) k_bp(BpArgs p)
 {
     if constexpr (GRP && bp_paired<VT>()) {
         const int g = 2 * (int)blockIdx.z + (int)(blockIdx.x & 1);
         if (g * SB >= p.S) return;
-        bp_tile<MODE, ST, VT, GRP, BULK>(p, blockIdx.x >> 1, blockIdx.y, g);
+        bp_tile<ST, VT, GRP>(p, blockIdx.x >> 1, blockIdx.y, g);
     } else {
-        bp_tile<MODE, ST, VT, GRP, BULK>(p, blockIdx.x, blockIdx.y, blockIdx.z);
+        bp_tile<ST, VT, GRP>(p, blockIdx.x, blockIdx.y, blockIdx.z);
     }
 }
 
@@ -1584,88 +1355,6 @@ __global__ void __launch_bounds__(512, RS < 2 ? 2 : 1) k_x_c2r(const float2* __r
                                                int packed, float* __restrict__ vol, size_t vol_slice)
 {
     x_c2r_block<RS>(w, Nx, Nz, plan, B, packed, vol, vol_slice, blockIdx.x, blockIdx.y);
-}
-
-// ---------------------------------------------------------------------------
-// Batched WBP: persistent stage kernels over many series.  A wave holds one
-// slab of every series in the batch (series of fewer slabs drop out of later
-// waves); each of the five WBP stages runs as one launch over the whole wave,
-// whose persistent CTAs pull virtual blocks — (series' slab, block of that
-// stage) — from a counter until none is left, and run the same block body
-// the per-series kernels run, so every result is bit-identical to the
-// per-series launches.
-// ---------------------------------------------------------------------------
-struct WbpSlab {
-    const float* proj;        // series projections [T][ny][nx]
-    size_t tilt_stride;
-    int row_pitch, y0;        // nx; first row of the slab
-    const float2* cs;
-    int T, N, Nx, Nz, S;
-    const float* h;           // R-weight transfer function
-    void* filt;               // staged, filtered sinogram (storage type of the batch)
-    float* scale;
-    int* flags;
-    float* g2;                // 2x grid, then the cropped spectrum
-    float2* y;                // row spectra
-    float* vol;               // the slab's first output slice
-    size_t vol_slice;
-    int b_rweight, b_row, b_xc2r, zcrop_cb, zcrop_pitch, packed;
-    float norm;
-    BpArgs bp;
-    FftPlan fN, f2x, f2z, fz, fx;
-    int gx[5];                // virtual grid x of each stage (y is the slab's slices; the BP's y, z below)
-    int bp_gy, bp_gz;
-};
-
-constexpr int kWbpStages = 5;   // rweight, bp, row_r2c, zcrop, x_c2r
-
-// Flags of every slab of the wave to zero (run_slab_t's memset); grid = slabs.
-__global__ void k_wave_flags(const WbpSlab* __restrict__ w)
-{
-    const WbpSlab& d = w[blockIdx.x];
-    for (int i = threadIdx.x; i < d.S; i += blockDim.x) d.flags[i] = 0;
-}
-
-// Stage STAGE of a wave: start[k] is the first virtual block of slab k
-// (start[nslabs] the total); counter starts at 0.
-template <int STAGE, typename ST, int RS>
-__global__ void __launch_bounds__(STAGE == 1 ? BP_THREADS : 512, STAGE == 1 ? 3 : (RS < 2 ? 2 : 1))
-    k_wbp_wave(const WbpSlab* __restrict__ w, const int* __restrict__ start, int nslabs, int* __restrict__ counter)
-{
-    __shared__ int s_item;
-    const int total = start[nslabs];
-    for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
-        __syncthreads();
-        const int item = s_item;
-        __syncthreads();
-        if (item >= total) return;
-        int lo = 0, hi = nslabs - 1;   // the slab whose block range holds item
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (start[mid] <= item) lo = mid;
-            else hi = mid - 1;
-        }
-        const WbpSlab& d = w[lo];
-        const int v = item - start[lo];
-        const int bx = v % d.gx[STAGE], by = v / d.gx[STAGE];
-        if constexpr (STAGE == 0) {
-            rweight_block<ST, RS>(d.proj, d.tilt_stride, d.row_pitch, d.y0, d.cs, d.T, d.N, d.Nz, d.h, d.fN,
-                                  d.b_rweight, static_cast<ST*>(d.filt), d.scale, d.flags, bx, by);
-        } else if constexpr (STAGE == 1) {
-            bp_tile<1, ST, float, false>(d.bp, bx, by % d.bp_gy, by / d.bp_gy);
-        } else if constexpr (STAGE == 2) {
-            row_r2c_block<RS>(d.g2, d.Nx, d.Nz, d.f2x, d.b_row, d.y, bx, by);
-        } else if constexpr (STAGE == 3) {
-            const float2* yv = d.y;
-            zcrop_block<RS>(yv, d.Nx, d.Nz, d.zcrop_cb, d.zcrop_pitch, d.f2z, d.fz, d.norm,
-                            reinterpret_cast<float2*>(d.g2), bx, by);
-        } else {
-            x_c2r_block<RS>(reinterpret_cast<const float2*>(d.g2), d.Nx, d.Nz, d.fx, d.b_xc2r, d.packed, d.vol,
-                            d.vol_slice, bx, by);
-        }
-        __syncthreads();   // shared memory is reused by the next block
-    }
 }
 
 }  // namespace at3r

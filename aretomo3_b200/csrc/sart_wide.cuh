@@ -26,7 +26,6 @@ namespace at3r {
 // infinity or a NaN: the blocked sums below multiply neighbouring samples by
 // zero weights, so such a slice takes the per-sample paths.  One bit per
 // producer, so that no kernel tests a bit that it sets itself.
-constexpr float kSpecial = 1e30f;
 
 constexpr int WIDE_THREADS = 256, WIDE_WARPS = WIDE_THREADS / 32;
 constexpr int FPW_RAYS = 2;                  // rays a thread carries
@@ -156,17 +155,6 @@ __device__ __forceinline__ void fpw_load(const float* even, const float* odd, fl
         v[2 * b] = make_float2(a.x, a.y);
         v[2 * b + 1] = make_float2(a.z, a.w);
     }
-}
-
-// Two FP32 fused multiply-adds in one instruction (the same rate per
-// multiply-add as the scalar form, half the issue slots).
-__device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b)
-{
-    unsigned long long r = *reinterpret_cast<unsigned long long*>(&acc);
-    asm("fma.rn.f32x2 %0, %1, %2, %0;"
-        : "+l"(r)
-        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
-    acc = *reinterpret_cast<float2*>(&r);
 }
 
 // ---------------------------------------------------------------------------
