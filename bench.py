@@ -193,16 +193,19 @@ def profiled_traffic(kernel: str, workload_name: str, storage: str):
     return d.get(f"{workload_name}/{storage}", {}).get(kernel)
 
 
-# Shared-memory / L1 bytes one work unit of a kernel moves on chip: the back-
-# projectors read one 8-byte (p[i], p[i+1]) pair per voxel, tilt and slice;
-# the forward projector reads four bilinear taps per ray sample and slice (a
-# 16-byte load serves four slices: 16 B per sample-slice, 8 B from the 16-bit
-# shadow).
+# Shared-memory bytes one work unit of a kernel moves on chip.  WBP back-
+# projection: three samples of a slice per block of four voxels.  FP32 SART: four
+# samples per block of four voxels; the forward projector reads, per ray
+# sample and slice, (1 + 2 sin + 2 cos) / 2 columns of a ray pair's window (1.8 on
+# average over +-60 degrees) and its share of their weights.  16-bit SART: an
+# 8-byte pair per voxel, four 2-byte taps per ray sample.
 def onchip_bytes_per_unit(kernel: str, storage: str):
-    if kernel in ("bp_sart", "bp_wbp_2x"):
-        return 8.0
+    if kernel == "bp_wbp_2x":
+        return 3.0
+    if kernel == "bp_sart":
+        return 4.0 if storage == "f32" else 8.0
     if kernel == "fp_diff":
-        return 16.0 if storage == "f32" else 8.0
+        return 8.1 if storage == "f32" else 8.0
     return None
 
 
