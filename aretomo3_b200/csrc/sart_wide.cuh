@@ -209,9 +209,12 @@ struct Fpw {
     static_assert(WARP_BYTES % 16 == 0, "16-byte aligned regions");
 };
 
-// The reference's ray of one slice, sample by sample with the empty test
-// (the path of slices that hold empty or non-finite voxels).
-__device__ __noinline__ float fpw_ray_tested(const float* v0, int E, int Nx, RayPos r, int lo, int hi, float* count)
+// The ray of one slice, sample by sample (the path of slices that hold empty,
+// infinite or NaN voxels): with the reference's empty test where the slice may hold
+// empty voxels; otherwise as the four-slice kernel sums it, with no difference of two taps,
+// so that a sample between infinite voxels is infinite and not NaN.
+__device__ __noinline__ float fpw_ray_tested(const float* v0, int E, int Nx, RayPos r, int lo, int hi, bool empty,
+                                             float* count)
 {
     float s = 0.f, n = 0.f;
     for (int i = lo; i <= hi; i++) {
@@ -219,9 +222,15 @@ __device__ __noinline__ float fpw_ray_tested(const float* v0, int E, int Nx, Ray
         const int iX = (int)fX, iZ = (int)fZ;
         const float* p = v0 + (ptrdiff_t)E * (iX - (ptrdiff_t)iZ * Nx);
         const ptrdiff_t row = (ptrdiff_t)E * Nx;
-        const float val = bilerp(__ldg(p), __ldg(p + E), __ldg(p - row), __ldg(p - row + E), fX - (float)iX, fZ - (float)iZ);
-        if (val < kSentinelTest) continue;
-        s += val;
+        const float a00 = __ldg(p), a10 = __ldg(p + E), a01 = __ldg(p - row), a11 = __ldg(p - row + E);
+        const float wx = fX - (float)iX, wz = fZ - (float)iZ, ux = 1.f - wx, uz = 1.f - wz;
+        if (empty) {
+            const float val = bilerp(a00, a10, a01, a11, wx, wz);
+            if (val < kSentinelTest) continue;
+            s += val;
+        } else {
+            s = __fmaf_rn(wx * wz, a11, __fmaf_rn(ux * wz, a01, __fmaf_rn(wx * uz, a10, __fmaf_rn(ux * uz, a00, s))));
+        }
         n += 1.f;
     }
     *count = n;
@@ -496,7 +505,7 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
 
     // mean along the ray, residual and R-factor sums
     float ad = 0.f, ar = 0.f;
-    unsigned tested = 0;   // slices whose samples are tested one by one
+    unsigned tested = 0, empty = 0;   // slices summed sample by sample; those of them with empty voxels
     int ys[NS / 4];
 #pragma unroll
     for (int k = 0; k < NS / 4; k++) {
@@ -504,8 +513,10 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
         const int4 f = __ldg(reinterpret_cast<const int4*>(p.flags + ys[k]));
         const int fl[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int q = 0; q < 4; q++) {
             if (fl[q] & (kFlagVolEmpty | kFlagRawSpecial | kFlagVolSpecial)) tested |= 1u << (4 * k + q);
+            if (fl[q] & kFlagVolEmpty) empty |= 1u << (4 * k + q);
+        }
     }
 #pragma unroll
     for (int r = 0; r < FPW_RAYS; r++) {
@@ -526,7 +537,8 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
             for (int q = 0; q < 4; q++) {
                 float sum = sums[q], cnt = n;
                 if ((tested >> (4 * b + q)) & 1)
-                    sum = fpw_ray_tested(p.vol + gvol + (size_t)(Nz - 1) * Nx * G + (ys[b] - g * G) + q, G, Nx, rp, lo, hi, &cnt);
+                    sum = fpw_ray_tested(p.vol + gvol + (size_t)(Nz - 1) * Nx * G + (ys[b] - g * G) + q, G, Nx, rp, lo, hi,
+                                         (empty >> (4 * b + q)) & 1, &cnt);
                 const float fp = cnt <= 0.f ? kSentinelValue : sum / cnt;
                 d[q] = 0.f;
                 if (!(fp < kSentinelTest) && !(rw[q] < kSentinelTest)) {
