@@ -121,6 +121,7 @@ struct at3r_plan {
     float* d_part = nullptr;                    // sums of the row segments
     int* d_arrived = nullptr;
     size_t n_arrived = 0;
+    int wait_polls = WIDE_POLLS;                // limit of its waits for bulk copies
     // host path
     float* d_proj_slab[2] = {nullptr, nullptr};
     float* d_vol_slab[2] = {nullptr, nullptr};
@@ -327,6 +328,7 @@ at3r_status run_sart_wide(at3r_plan* p, const float* proj, size_t tilt_stride, i
     AT3R_CUDA(cudaMemsetAsync(w, 0, sizeof(float) * (size_t)SG * G * Nx * Nz, st));
     BpwArgs b{};
     b.cs = p->d_cs; b.vol = w; b.flags = p->d_flags; b.T = T; b.N = N; b.Nx = Nx; b.Nz = Nz;
+    b.polls = p->wait_polls;
     const dim3 bgrid((Nx + bpw_tile_x<LP>() - 1) / bpw_tile_x<LP>(), (Nz + BPW_TILE_Z - 1) / BPW_TILE_Z, SG);
     // first back-projection: all tilts, relax 1 (CTomoSart.cpp:68-69)
     b.sino = raw; b.t0 = 0; b.t1 = T; b.relax = 1.f; b.low_bit = kFlagRawLow;
@@ -338,6 +340,7 @@ at3r_status run_sart_wide(at3r_plan* p, const float* proj, size_t tilt_stride, i
     f.vol = w; f.raw = raw; f.diff = dif; f.cs = p->d_cs; f.flags = p->d_flags;
     f.Nx = Nx; f.Nz = Nz; f.S = S; f.T = T; f.N = N;
     f.part = p->d_part; f.arrived = p->d_arrived; f.seg_rows = p->fp_seg_rows;
+    f.polls = p->wait_polls;
     const int blocks = (N + FPW_CTA_RAYS - 1) / FPW_CTA_RAYS, segs = (Nz + f.seg_rows - 1) / f.seg_rows;
     AT3R_CUDA(cudaMemsetAsync(p->d_arrived, 0, sizeof(int) * p->n_arrived, st));
     for (int it = 0; it < p->g.iterations; it++) {
@@ -542,7 +545,8 @@ at3r_status begin_run(at3r_plan* p, cudaStream_t st)
     int dev = -1;
     AT3R_CUDA(cudaGetDevice(&dev));
     if (dev != p->device) return set_err(AT3R_ERR_INVALID_ARGUMENT, "plan was created on another device");
-    AT3R_CUDA(cudaMemsetAsync(p->d_seen, 0, sizeof(int), st));
+    at3r_status rc = at3r_plan_clear_seen(p, st);
+    if (rc) return rc;
     if (p->g.method == AT3R_SART && p->g.compute_rfactor)
         AT3R_CUDA(cudaMemsetAsync(p->d_rf, 0, sizeof(double) * 2 * std::max(1, p->g.iterations), st));
     return AT3R_OK;
@@ -557,6 +561,24 @@ at3r_status end_run(at3r_plan* p, cudaStream_t st)
 }
 
 }  // namespace
+
+at3r_status at3r_plan_clear_seen(at3r_plan* p, cudaStream_t st)
+{
+    AT3R_CUDA(cudaMemsetAsync(p->d_seen, 0, sizeof(int), st));
+    return AT3R_OK;
+}
+
+at3r_status at3r_plan_finish(at3r_plan* p, cudaStream_t st)
+{
+    int seen = 0;
+    if (p->wide) AT3R_CUDA(cudaMemcpyAsync(&seen, p->d_seen, sizeof(int), cudaMemcpyDeviceToHost, st));
+    AT3R_CUDA(cudaStreamSynchronize(st));
+    if (seen & kFlagStageTimeout)
+        return set_err(AT3R_ERR_CUDA, "a SART kernel gave up waiting for a bulk copy: the volume is not valid");
+    return AT3R_OK;
+}
+
+extern "C" void at3r_plan_set_wait_polls(at3r_plan* p, int polls) { p->wait_polls = polls; }
 
 cudaMemPool_t at3r_device_pool(int dev)
 {
@@ -1300,8 +1322,7 @@ at3r_status run_host_body(at3r_plan* p, const float* const* frames, float* const
     if (!out_pinned && (rc = drain_out(nslab - 1))) return rc;
     AT3R_CUDA(cudaStreamWaitEvent(st, p->ev[4 + ((nslab - 1) & 1)], 0));
     if ((rc = end_run(p, st))) return rc;
-    AT3R_CUDA(cudaStreamSynchronize(st));
-    return AT3R_OK;
+    return at3r_plan_finish(p, st);
 }
 
 at3r_status run_host_impl(at3r_plan* p, const float* const* frames, float* const* vol_frames, float* vol_xyz,

@@ -14,6 +14,14 @@ size_t at3r_estimate_resident_bytes(const at3r_geom* g, int* slab_out);
 // One slab of a device-resident series proj[T][ny][nx]: rows [y0, y0 + n)
 // into vol_rows[n][Nz][Nx] on `st`, without the per-run bookkeeping.
 at3r_status at3r_plan_run_slab(at3r_plan* p, const float* proj, int y0, int n, float* vol_rows, cudaStream_t st);
+// For callers of at3r_plan_run_slab: clears what the plan's runs met, before
+// the first slab, and after the last one waits for `st` and returns an error
+// if a kernel gave up waiting for a bulk copy (its volume is not valid).
+at3r_status at3r_plan_clear_seen(at3r_plan* p, cudaStream_t st);
+at3r_status at3r_plan_finish(at3r_plan* p, cudaStream_t st);
+// Polls after which the SART kernels give up waiting for a bulk copy; 0: at
+// once (tests of the error path).
+extern "C" void at3r_plan_set_wait_polls(at3r_plan* p, int polls);
 // Sets the calling thread's at3r_last_error() text.
 void at3r_set_last_error(const char* msg);
 // The library's device memory pool of device `dev` (freed blocks stay cached

@@ -130,6 +130,12 @@ bool start_request(Request* r)
         r->err = at3r_last_error();
         return false;
     }
+    rc = at3r_plan_clear_seen(r->plan, r->st);
+    if (rc != AT3R_OK) {
+        r->status = rc;
+        r->err = at3r_last_error();
+        return false;
+    }
     const size_t T = r->g.n_tilts, ny = r->g.ny, nx = r->g.nx, Nx = nx & ~1, Nz = r->g.vol_z;
     const size_t frame = ny * nx, vslab = (size_t)r->slab * Nx * Nz;
     e = cudaMallocAsync(reinterpret_cast<void**>(&r->d_proj), sizeof(float) * T * frame, r->st);
@@ -348,7 +354,12 @@ void engine_main(at3r_server* s)
                 if (!issue_slab(r, level, s->prio_greatest + level)) break;
                 moved = true;
             }
-            if (r->status != AT3R_OK || (r->rows_done == r->g.ny && r->inflight.empty())) {
+            const bool done = r->rows_done == r->g.ny && r->inflight.empty();
+            if (r->status == AT3R_OK && done) {
+                r->status = at3r_plan_finish(r->plan, r->last);
+                if (r->status != AT3R_OK) r->err = at3r_last_error();
+            }
+            if (r->status != AT3R_OK || done) {
                 finish(s, r);
                 active.erase(active.begin() + (long)i);
                 moved = true;

@@ -374,7 +374,7 @@ __device__ __forceinline__ float bp_xp(float fX, float fZs, float c, float cent)
     return __fadd_rn(__fmaf_rn(a, 0.5f, cent), 0.5f);
 }
 
-constexpr int kFlagStageTimeout = 16;   // a bulk copy did not arrive (the output was not written)
+constexpr int kFlagStageTimeout = 16;   // a bulk copy did not arrive: the volume is not valid
 
 __host__ __device__ inline size_t bp_smem_bytes()
 {

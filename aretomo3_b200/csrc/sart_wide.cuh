@@ -33,6 +33,7 @@ constexpr int FPW_LP = 4;                    // lanes that share its rays
 constexpr int FPW_WARP_RAYS = FPW_RAYS * 32 / FPW_LP, FPW_PAIRS = 32 / FPW_LP;
 constexpr int FPW_MAX_COLS = 32;             // columns of a ray pair's window; wider (steeper than ~83 degrees): per sample
 constexpr int FPW_MAX_ROWS = 8;              // volume rows per weight table
+constexpr int WIDE_POLLS = 1 << 22;          // polls of a wait for a bulk copy before it gives up
 
 // Back-projector: slices of a thread, NS = 8 as two runs of four at 4 LP k + 4 lp
 // (each 16-byte load of the LP lanes is contiguous).
@@ -192,6 +193,7 @@ struct FpwArgs {
     int* arrived;            // [group][nt][ray warps]: segments done; zero between launches
     int seg_rows;            // volume rows a warp walks
     int Nx, Nz, S, T, N, t0, nt;
+    int polls;               // limit of a wait for a bulk copy (WIDE_POLLS)
 };
 
 constexpr int FPW_THREADS = 128, FPW_WARPS = FPW_THREADS / 32, FPW_CTA_RAYS = FPW_WARPS * FPW_WARP_RAYS;
@@ -392,8 +394,9 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
                 }
                 __syncwarp();
             }
-            for (int j = 0; j < nr; j++) {
-                ok = mbar_wait(bar0 + 8 * sc, phase, 1 << 22);
+            int j = 0;
+            for (; j < nr; j++) {
+                ok = mbar_wait(bar0 + 8 * sc, phase, p.polls);
                 if (!__all_sync(0xffffffffu, ok)) break;
                 const float* v = reinterpret_cast<const float*>(region + sc * row_bytes) + s_off[j * FPW_PAIRS + pair];
                 const float2* w = tab + (j * FPW_PAIRS + pair) * CP;
@@ -426,10 +429,21 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
                       in ? row.bytes : next.bytes);
                 if (++sc == ns) { sc = 0; phase ^= 1; }
             }
-            if (!__all_sync(0xffffffffu, ok)) {   // a copy did not arrive: wait once more (bounded), flag the slices, write nothing
-                for (int k = 0; k < ns; k++) mbar_wait(bar0 + 8 * k, phase, 1 << 22);
+            if (!__all_sync(0xffffffffu, ok)) {
+                // a copy did not arrive: the run is flagged.  Row zc + j and the rows fetched ahead of it are
+                // in flight, in the stages from sc on, the parity changing where the ring starts over: wait
+                // for each (bounded), so that none lands in another CTA's memory.  The warp's sums become
+                // zero and it goes on, so that the segments of its rays still count up to their last one
+                for (int k = 0; k < lead && zc + j + k <= z1; k++) {
+                    const int sg = sc + k;
+                    mbar_wait(bar0 + 8 * (sg < ns ? sg : sg - ns), sg < ns ? phase : phase ^ 1, WIDE_POLLS);
+                }
                 if (lane == 0) atomicOr(p.flags + g * G, kFlagStageTimeout);
-                return;
+#pragma unroll
+                for (int r = 0; r < FPW_RAYS; r++)
+#pragma unroll
+                    for (int q = 0; q < NS / 2; q++) acc[r][q] = make_float2(0.f, 0.f);
+                break;
             }
             row = next;
         }
@@ -582,6 +596,7 @@ struct BpwArgs {
     float* vol;              // W
     int* flags;
     int T, N, t0, t1, Nx, Nz, low_bit;
+    int polls;               // limit of a wait for a bulk copy (WIDE_POLLS)
     float relax;
 };
 
@@ -696,7 +711,13 @@ __global__ void __launch_bounds__(WIDE_THREADS, 3) k_bp_wide(BpwArgs p)
     bool ok = true;
     uint32_t phase = 0;
     for (int tc = p.t0, b = 0; tc < p.t1; tc += BPW_CHUNK) {
-        ok = ok && mbar_wait(smem_u32(mbar + b), phase, 1 << 22);
+        if (ok && !mbar_wait(smem_u32(mbar + b), phase, p.polls)) {
+            // a window did not arrive: wait (bounded) for this chunk's copies and, where there is
+            // a next chunk, its own, which are in flight too (buffer 0 of it is a phase on)
+            ok = false;
+            mbar_wait(smem_u32(mbar + b), phase, WIDE_POLLS);
+            if (tc + BPW_CHUNK < p.t1) mbar_wait(smem_u32(mbar + (b ^ 1)), b ? phase ^ 1 : phase, WIDE_POLLS);
+        }
         const int nc = min(BPW_CHUNK, p.t1 - tc);
         for (int j = 0; j < nc; j++) {
             const int kw = s_kw[b * BPW_CHUNK + j];
@@ -745,15 +766,16 @@ __global__ void __launch_bounds__(WIDE_THREADS, 3) k_bp_wide(BpwArgs p)
         }
         if (b) phase ^= 1;
         if (tc + 2 * BPW_CHUNK < p.t1) {
-            __syncthreads();   // the buffer is free
+            // the buffer is free; nothing more is fetched once a wait of any thread ran out
+            if (!__syncthreads_and(ok)) { ok = false; break; }
             fetch(tc + 2 * BPW_CHUNK, b);
             __syncthreads();   // s_kw
         }
         b ^= 1;
     }
-    ok = ok && mbar_wait(smem_u32(mbar + 2), 0, 1 << 22);
-    if (!ok) {   // a copy did not arrive: wait once more (bounded), flag the slices, write nothing
-        for (int k = 0; k < 3; k++) mbar_wait(smem_u32(mbar + k), k < 2 ? phase : 0, 1 << 22);
+    ok = ok && mbar_wait(smem_u32(mbar + 2), 0, p.polls);
+    if (!ok) {   // a copy did not arrive: the run is flagged, the voxels keep their values
+        mbar_wait(smem_u32(mbar + 2), 0, WIDE_POLLS);
         atomicOr(p.flags + g * G, kFlagStageTimeout);
         return;
     }

@@ -255,7 +255,9 @@ class Plan:
     def flags_seen(self) -> int:
         """Bits of what the last run met (at3r_plan_flags_seen): 1 empty SART
         voxels (filled), 2 staged projections near the missing-value test, 4
-        the residual near it, 8 a fill chain took the slice mean."""
+        the residual near it, 8 a fill chain took the slice mean, 16 a kernel
+        gave up waiting for a bulk copy and the volume is not valid (run_host,
+        DoIt and the server raise then; run_device does not wait, so look here)."""
         v = int(lib().at3r_plan_flags_seen(self._h))
         if v < 0:
             _check(2)

@@ -138,7 +138,9 @@ int at3r_plan_c2r(const at3r_plan* plan);
  * held values at or below -5e9 (near the -1e10 "missing" test), so the
  * back-projection tested every sample; 4 the SART residual did; 8 a fill chain
  * found no non-empty voxel and took the slice mean; 16 a SART kernel gave up
- * waiting for a bulk copy and did not write its output.  -1 on a CUDA error. */
+ * waiting for a bulk copy, so the volume is not valid: the host forms and the
+ * serving loop return AT3R_ERR_CUDA then, and callers of the device and batched
+ * forms, which do not wait, look here.  -1 on a CUDA error. */
 int at3r_plan_flags_seen(const at3r_plan* plan);
 /* The SART plan's fill table (see at3r_geom.fill_seed): Nx * Nz entries, entry
  * i = Z * Nx + X for the voxel at (X, Z) of a slice before the z flip, as

@@ -5,6 +5,8 @@ against the FP64 oracle.
 Tolerance: a value is a few thousand FP32 multiply-adds, so its relative error
 is about sqrt(n) * 2^-24 ~ 4e-6 of the volume's scale; 2e-5 leaves the
 few iterations' worth of room."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -100,3 +102,31 @@ def test_an_unusual_row_equals_the_four_slice_kernels(bad, ny):
         ref, rseen = _run(np.ascontiguousarray(f[:, y0:y0 + 4]), tilts, 32, iterations=2, subsets=4)
         _same_values(vol[y], ref[y - y0], TOL)
         assert rseen & ~seen == 0, "a condition of the row was not seen"
+
+
+@pytest.mark.parametrize("ny,nz", [(30, 24), (64, 90)])
+def test_a_wait_that_runs_out_is_an_error(ny, nz):
+    """With a limit of no polls every wait for a bulk copy gives up: the host form returns an
+    error and the run is flagged.  With the limit back, the same plan gives the bits it gave
+    before (no copy and no count of the failed run is left over)."""
+    from aretomo3_b200 import recon
+    tilts = np.linspace(-60, 60, 21).astype(np.float32)
+    f = _series(140, ny, tilts, nz, seed=8)
+    plan = recon.Plan(140, ny, tilts, nz, method=recon.SART, fill_seed=3, iterations=2, subsets=3)
+    set_polls = recon.lib().at3r_plan_set_wait_polls
+    set_polls.argtypes, set_polls.restype = [ctypes.c_void_p, ctypes.c_int], None
+    try:
+        def run():
+            vol = np.empty(plan.volume_shape, np.float32)
+            plan.run_host([f[t] for t in range(tilts.size)], [vol[y] for y in range(ny)])
+            return vol
+        ref = run()
+        set_polls(plan._h, 0)
+        with pytest.raises(recon.ReconError, match="bulk copy"):
+            run()
+        assert plan.flags_seen() & 16
+        set_polls(plan._h, 1 << 22)
+        assert np.array_equal(run(), ref)
+        assert not plan.flags_seen() & 16
+    finally:
+        plan.close()
