@@ -628,7 +628,8 @@ static size_t wide_subset(const at3r_geom* g)
 // volume.  It follows the series, not the slab (the segments' sums are part of a result).
 static int wide_seg_rows(const at3r_geom* g)
 {
-    const long N = g->nx & ~1, warps = (N + 15) / 16 * (long)wide_subset(g) * ((g->ny + 63) / 64);
+    // (at least one ray: the size estimates are asked about widths that no plan accepts)
+    const long N = std::max(g->nx & ~1, 2), warps = (N + 15) / 16 * (long)wide_subset(g) * ((g->ny + 63) / 64);
     const long segs = std::max((long)(g->vol_z + 319) / 320, std::min((long)(2 * 8 * 148 + warps - 1) / warps, (long)g->vol_z / 24));
     return (int)((g->vol_z + std::max(segs, 1L) - 1) / std::max(segs, 1L));
 }
@@ -666,7 +667,7 @@ int default_slab(const at3r_geom* g, int sms)
     const size_t per_slice = slice_bytes(g);
     long S;
     if (g->method == AT3R_SART) {
-        const long N = g->nx & ~1;
+        const long N = std::max(g->nx & ~1, 2);
         const long nt = std::max(1, (g->num_tilts + g->subsets - 1) / std::max(1, g->subsets));
         const long per_group = ((N + 255) / 256) * nt;
         const long target = (long)sms * 6 * 16;

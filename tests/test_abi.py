@@ -3,6 +3,8 @@ include/at3r.h declares, and rejects invalid geometry before touching a GPU."""
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -74,6 +76,19 @@ def test_estimate_bytes_without_gpu():
     big = recon.estimate_bytes(4096, 4096, tilts, 1200, method=recon.SART, storage=recon.STORE_F16)
     assert big > 2 * 8 * 4096 * 1200 * 4
     assert recon.estimate_bytes(0, 64, tilts, 64) == 0
+
+
+@pytest.mark.parametrize("method,storage", [(0, 0), (1, 0), (1, 1), (1, 2)])
+def test_estimate_bytes_of_the_narrowest_series(method, storage):
+    """A width below the four columns a plan wants must not end the process (one column
+    leaves no ray to divide by); a size that no plan accepts may be estimated as anything."""
+    code = ("import sys; sys.path.insert(0, %r); from aretomo3_b200 import recon\n"
+            "for nx in (1, 2, 3, 4, 5):\n"
+            "    for ny in (1, 4, 30, 64):\n"
+            "        b = recon.estimate_bytes(nx, ny, [-30, 0, 30], 64, method=%d, storage=%d, subsets=3)\n"
+            "        assert nx < 4 or b > 0" % (ROOT, method, storage))
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+    assert out.returncode == 0, (out.returncode, out.stderr)
 
 
 def test_reproj_range_matches_oracle_without_gpu():
