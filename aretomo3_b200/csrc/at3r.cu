@@ -612,9 +612,12 @@ at3r_status at3r_plan_create(const at3r_geom* g, at3r_plan** out) { return plan_
 // 15.5 against 17.1) and stay.  It follows the series, not the slab, so that a slab size
 // never changes a result.
 constexpr double kWideFill = 1.3;
+// Their grids have the volume rows and the tilts in y; longer series keep the four-slice kernels.
+constexpr int kWideMaxY = 65535;
 static bool sart_wide(const at3r_geom* g)
 {
-    return g->method == AT3R_SART && g->storage == AT3R_STORE_F32 && wide_cost(g->ny) <= kWideFill * g->ny;
+    return g->method == AT3R_SART && g->storage == AT3R_STORE_F32 && wide_cost(g->ny) <= kWideFill * g->ny &&
+           g->vol_z <= kWideMaxY && g->n_tilts <= kWideMaxY;
 }
 
 // The most tilts of a subset.

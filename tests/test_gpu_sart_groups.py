@@ -130,3 +130,16 @@ def test_a_wait_that_runs_out_is_an_error(ny, nz):
         assert not plan.flags_seen() & 16
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("nx,nz,T", [(8, 65535, 5), (8, 65537, 5), (4, 6, 65535), (4, 6, 65600)])
+def test_sizes_around_the_grid_limits(nx, nz, T):
+    """Thickness and tilt count at the largest y extent of a grid and past it, against the FP64
+    oracle.  A serial FP32 sum of n nearly equal terms (the samples of a ray, the tilts
+    of a voxel) can round the same way throughout: n * 2^-25 of itself."""
+    tilts = np.linspace(-50, 50, T).astype(np.float32)
+    f = np.random.default_rng(T).normal(50, 5, (T, 32, nx)).astype(np.float32)
+    vol, seen = _run(f, tilts, nz, iterations=1, subsets=3)
+    assert not seen & 16
+    ref = sart(np.ascontiguousarray(f[:, 4:6]), tilts, nz, 0, T, 1, 3, threads=1)
+    assert rel_l2(vol[4:6], ref) < max(nz, T) * 2.0 ** -25
