@@ -76,3 +76,23 @@ def test_an_unusual_row_leaves_the_others_alone(bad):
     same = [y for y in range(9) if y != 5]
     assert np.array_equal(vol[same], ref[same])
     assert not np.array_equal(vol[5], ref[5], equal_nan=True)
+
+
+def _unusual(bad, ny):
+    tilts = np.linspace(-60, 60, 19).astype(np.float32)
+    f = _series(96, ny, tilts, 40, seed=4)
+    f[2, ny - 1, 30] = bad
+    f[7, ny - 1, 90] = bad
+    return f, tilts
+
+
+@pytest.mark.parametrize("ny", [3, 9])
+@pytest.mark.parametrize("bad", [4e12, -4e12])
+def test_an_unusual_row_equals_the_oracle(bad, ny):
+    """The oracle's means of the samples above -1e10.  The filter makes samples of some 1e11 of the
+    pixel, so that FP32 errors of 1e4 leave no sample on the other side of the test but one
+    within 1e-6 of it: a voxel of the 2x grid, 1e-4 of the scale."""
+    f, tilts = _unusual(bad, ny)
+    vol, mode = _run(f, tilts, 40)
+    y = ny - 1
+    assert rel_l2(vol[y], wbp(f, tilts, 40, y0=y, y1=y + 1, c2r_mode=mode)[0]) < 1e-4
