@@ -64,8 +64,10 @@ __device__ __forceinline__ void wbp_span(float2 c, int X0, int Z0, float hx, flo
 }
 
 // Windows of tilts [c0, c0 + nc) of slices [ys, ys + n), n <= 4, into win[nc][WBP_WW]; zero off the detector.
-template <typename ST>
-__device__ __forceinline__ void wbp_stage(const WbpBpArgs& p, float4* win, const int* ws, int c0, int nc, int ys, int n)
+// NAN_STAYS: slices of the mask `nan` keep a stored NaN, the 16-bit types' code of a missing value.
+template <typename ST, bool NAN_STAYS = false>
+__device__ __forceinline__ void wbp_stage(const WbpBpArgs& p, float4* win, const int* ws, int c0, int nc, int ys, int n,
+                                          unsigned nan = 0)
 {
     for (int e = threadIdx.x; e < nc * WBP_WW; e += WBP_THREADS) {
         const int t = e / WBP_WW, x = ws[t] + (e - t * WBP_WW);
@@ -74,9 +76,11 @@ __device__ __forceinline__ void wbp_stage(const WbpBpArgs& p, float4* win, const
         for (int q = 0; q < 4; q++) {
             const size_t row = (size_t)(ys + q) * p.T + c0 + t;
             v[q] = 0.f;
-            if (q < n && x >= 0 && x < p.N)
-                v[q] = Stor<ST>::ld(static_cast<const ST*>(p.sino) + row * p.N + x,
-                                    std::is_same<ST, float>::value ? 1.f : __ldg(p.scale + row));
+            if (q < n && x >= 0 && x < p.N) {
+                const ST* src = static_cast<const ST*>(p.sino) + row * p.N + x;
+                const float sc = std::is_same<ST, float>::value ? 1.f : __ldg(p.scale + row);
+                v[q] = NAN_STAYS && ((nan >> q) & 1) ? static_cast<float>(__ldg(src)) * sc : Stor<ST>::ld(src, sc);
+            }
         }
         win[e] = make_float4(v[0], v[1], v[2], v[3]);
     }
@@ -99,6 +103,10 @@ __device__ __noinline__ void wbp_quad_tested(const WbpBpArgs& p, int bx, int by,
     const int X0 = bx * WBP_T, Z0 = by * WBP_T, X = wbp_x(X0, warp, lane), Z = wbp_z(Z0, warp, lane);
     const float cent = (float)(p.N / 2), endX = (float)(p.N - 2);
     const float hx = (float)p.GX / 2.0f, hz = (float)p.GZ / 2.0f;
+    // a slice with no value near the empty marker holds no missing value: its NaNs are NaNs
+    unsigned nan = 0;
+    for (int q = 0; q < n; q++)
+        if (!(__ldg(p.flags + ys + q) & kFlagRawLow)) nan |= 1u << q;
     float sum[4][4], cnt[4][4];   // [voxel 2 dz + dx][slice]
 #pragma unroll
     for (int v = 0; v < 4; v++)
@@ -114,7 +122,7 @@ __device__ __noinline__ void wbp_quad_tested(const WbpBpArgs& p, int bx, int by,
             cs_s[tid] = c;
         }
         __syncthreads();
-        wbp_stage<ST>(p, win, ws, c0, nc, ys, n);
+        wbp_stage<ST, true>(p, win, ws, c0, nc, ys, n, nan);
         __syncthreads();
         for (int t = 0; t < nc; t++) {
             const float2 c = cs_s[t];

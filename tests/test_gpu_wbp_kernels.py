@@ -87,6 +87,19 @@ def _unusual(bad, ny):
 
 
 @pytest.mark.parametrize("ny", [3, 9])
+@pytest.mark.parametrize("storage", [0, 1, 2])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_a_pixel_that_is_not_finite_leaves_no_value_of_its_row(bad, storage, ny):
+    """The R-weighting spreads it over its tilt's row and the crop over the slice: NaN, not a
+    reconstruction without that tilt (a stored NaN is the 16-bit types' code of a missing value,
+    but no value here is one)."""
+    f, tilts = _unusual(bad, ny)
+    vol, _ = _run(f, tilts, 40, storage=storage)
+    assert np.isnan(vol[ny - 1]).all()
+    assert np.isfinite(vol[:ny - 1]).all()
+
+
+@pytest.mark.parametrize("ny", [3, 9])
 @pytest.mark.parametrize("bad", [4e12, -4e12])
 def test_an_unusual_row_equals_the_oracle(bad, ny):
     """The oracle's means of the samples above -1e10.  The filter makes samples of some 1e11 of the
