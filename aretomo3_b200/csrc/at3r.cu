@@ -413,6 +413,8 @@ at3r_status run_slab_t(at3r_plan* p, const float* proj, size_t tilt_stride, int 
         switch (wide_group(S)) {
             case 64: rc = run_sart_wide<8, 8>(p, proj, tilt_stride, proj_y0, S, vol, st); break;
             case 32: rc = run_sart_wide<8, 4>(p, proj, tilt_stride, proj_y0, S, vol, st); break;
+            case 8: rc = run_sart_wide<2, 4>(p, proj, tilt_stride, proj_y0, S, vol, st); break;
+            case 4: rc = run_sart_wide<1, 4>(p, proj, tilt_stride, proj_y0, S, vol, st); break;
             default: rc = run_sart_wide<4, 4>(p, proj, tilt_stride, proj_y0, S, vol, st); break;
         }
         return rc != AT3R_OK ? rc : run_fill(p, S, vol, st);
@@ -616,7 +618,7 @@ constexpr double kWideFill = 1.3;
 constexpr int kWideMaxY = 65535;
 static bool sart_wide(const at3r_geom* g)
 {
-    return g->method == AT3R_SART && g->storage == AT3R_STORE_F32 && wide_cost(g->ny) <= kWideFill * g->ny &&
+    return g->method == AT3R_SART && g->storage == AT3R_STORE_F32 && wide_cost(g->ny, 16) <= kWideFill * g->ny &&
            g->vol_z <= kWideMaxY && g->n_tilts <= kWideMaxY;
 }
 
@@ -636,10 +638,10 @@ static int wide_seg_rows(const at3r_geom* g)
     const long segs = std::max((long)(g->vol_z + 319) / 320, std::min((long)(2 * 8 * 148 + warps - 1) / warps, (long)g->vol_z / 24));
     return (int)((g->vol_z + std::max(segs, 1L) - 1) / std::max(segs, 1L));
 }
-// Counters of the segments: one per group of 16 or more slices, tilt and 16 or more rays.
+// Counters of the segments: one per group of four or more slices, tilt and 16 rays.
 static size_t wide_arrived(const at3r_geom* g, int slices)
 {
-    return (size_t)((slices + 15) / 16) * wide_subset(g) * (size_t)(((g->nx & ~1) + 15) / 16);
+    return (size_t)((slices + 3) / 4) * wide_subset(g) * (size_t)(((g->nx & ~1) + 15) / 16);
 }
 
 // Workspace bytes one slice adds: SART two staged rows per tilt, the working
@@ -816,6 +818,10 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
             for (auto& f : {std::make_pair((const void*)k_fp_wide<64>, Fpw<64>::SMEM),
                             std::make_pair((const void*)k_fp_wide<32>, Fpw<32>::SMEM),
                             std::make_pair((const void*)k_fp_wide<16>, Fpw<16>::SMEM),
+                            std::make_pair((const void*)k_fp_wide<8>, Fpw<8>::SMEM),
+                            std::make_pair((const void*)k_fp_wide<4>, Fpw<4>::SMEM),
+                            std::make_pair((const void*)k_bp_wide<2, 4>, bpw_smem<2, 4>()),
+                            std::make_pair((const void*)k_bp_wide<1, 4>, bpw_smem<1, 4>()),
                             std::make_pair((const void*)k_bp_wide<8, 8>, bpw_smem<8, 8>()),
                             std::make_pair((const void*)k_bp_wide<8, 4>, bpw_smem<8, 4>()),
                             std::make_pair((const void*)k_bp_wide<4, 4>, bpw_smem<4, 4>())})

@@ -4,7 +4,7 @@
 // voxel or a ray serve all slices.  Here the slices are the innermost index:
 //   volume    W[group][Nz][Nx][G]   rows z flipped, G slices of a group
 //   sinogram  R[group][T][N][G]     weighted rows and residual
-// with G = 16, 32 or 64: a few lanes share a position and carry its G slices, read
+// with G = 16, 32 or 64 (slabs of fewer slices: 8 or 4): a few lanes share a position and carry its G slices, read
 // as contiguous runs.  Every load is then fully coalesced whatever the tilt (with
 // rays or voxels on the lanes, a warp's samples lie 1/cos or cos apart and a
 // 16-byte tap load took 6.6 to 8.1 wavefronts for 4), and a thread that carries a
@@ -49,7 +49,7 @@ __device__ __forceinline__ int bpw_slice(int lp, int k)
 template <int NS>
 __device__ __forceinline__ int fpw_slice(int lp, int pair, int b)
 {
-    return NS == 4 ? 4 * lp : 16 * (b ^ (pair & 1)) + 4 * lp;
+    return NS <= 4 ? NS * lp : 16 * (b ^ (pair & 1)) + 4 * lp;
 }
 
 // Columns that rays up to d detector samples apart can touch in one volume row of
@@ -117,11 +117,16 @@ __global__ void __launch_bounds__(256) k_ungroup_wide(const float* __restrict__ 
 // Group size for a slab of S slices: the cheapest once the last group is filled up.  Time
 // per slice against G = 64, measured on 4096 x 64 x 41 and 1024 x 256 x 61
 // reconstructions: 1.18 for 32 (fewer slices share a weight and a position), 1.65 for 16.
-inline double wide_cost(int S, int* group = nullptr)
+// From `smallest` on: 16 for a series; a slab of fewer slices also takes 8 (2.6 and 3.2) and 4
+// (4.8 and 6.2), so that slab_slices of a few slices costs neither the work nor the memory
+// of 16.  Measured (2 iterations of 4096 x 64 x 41 x 1200; four-slice kernels / filled
+// up to 16 / now): slabs of 1 slice 377 / 729 / 486 ms, of 4 97 / 182 / 122, of 8 63 / 91 / 65;
+// 2048 x 32 x 41 x 600, 3 iterations: of 4 29.2 / - / 27.6, of 8 16.5 / - / 14.3.
+inline double wide_cost(int S, int smallest, int* group = nullptr)
 {
-    const double rate[3] = {1.0, 1.18, 1.65};
+    const double rate[5] = {1.0, 1.18, 1.65, 2.8, 5.2};
     double best = 1e30;
-    for (int k = 0; k < 3; k++) {
+    for (int k = 0; 64 >> k >= smallest; k++) {
         const int G = 64 >> k;
         const double c = rate[k] * ((S + G - 1) / G * G);
         if (c < best) {
@@ -134,22 +139,43 @@ inline double wide_cost(int S, int* group = nullptr)
 inline int wide_group(int S)
 {
     int G = 64;
-    wide_cost(S, &G);
+    wide_cost(S, 4, &G);
     return G;
 }
-// Slices the workspace holds for slabs of up to S, filled-up groups included.
+// Slices the workspace holds for slabs of up to S, filled-up groups included (a slab of 64
+// slices fewer is no larger, filled up, than one that is not filled up at all).
 inline int wide_slices(int S)
 {
-    int m = 0;
-    for (int s = 1; s <= S; s++) m = std::max(m, (s + wide_group(s) - 1) / wide_group(s) * wide_group(s));
+    int m = S;
+    for (int s = std::max(1, S - 63); s <= S; s++) m = std::max(m, (s + wide_group(s) - 1) / wide_group(s) * wide_group(s));
     return m;
+}
+
+// V = 4, 2 or 1 values in one access.
+template <int V>
+using VecOf = std::conditional_t<V == 4, float4, std::conditional_t<V == 2, float2, float>>;
+template <int V>
+__device__ __forceinline__ void unpack(const VecOf<V>& a, float (&v)[V])
+{
+    if constexpr (V == 4) { v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; }
+    else if constexpr (V == 2) { v[0] = a.x; v[1] = a.y; }
+    else v[0] = a;
+}
+template <int V>
+__device__ __forceinline__ VecOf<V> pack(const float (&v)[V])
+{
+    if constexpr (V == 4) return make_float4(v[0], v[1], v[2], v[3]);
+    else if constexpr (V == 2) return make_float2(v[0], v[1]);
+    else return v[0];
 }
 
 // NS slices of one column in pairs of slices; even: the address of the lane's part of its
 // pair's first chunk, odd: of the second (fpw_slice).
 template <int NS>
-__device__ __forceinline__ void fpw_load(const float* even, const float* odd, float2 (&v)[NS / 2])
+__device__ __forceinline__ void fpw_load(const float* even, const float* odd, float2 (&v)[(NS + 1) / 2])
 {
+    if constexpr (NS == 2) v[0] = *reinterpret_cast<const float2*>(even);
+    if constexpr (NS == 1) v[0] = make_float2(*even, 0.f);
 #pragma unroll
     for (int b = 0; b < NS / 4; b++) {
         const float4 a = *reinterpret_cast<const float4*>((b & 1 ? odd : even) + 32 * (b >> 1));
@@ -207,7 +233,7 @@ struct Fpw {
     static constexpr int TABLE = G == 64 ? 5 << 10 : 3 << 10;
     static constexpr int WARP_BYTES = RING + TABLE + 8 * FPW_MAX_STAGES + 8 * FPW_MAX_ROWS * FPW_PAIRS + 4 * FPW_MAX_ROWS;
     static constexpr size_t SMEM = (size_t)FPW_WARPS * WARP_BYTES;
-    static constexpr int CTAS = G == 64 ? 2 : 4;
+    static constexpr int CTAS = G == 64 ? 2 : G >= 16 ? 4 : 5;   // (G 4 and 8: 2 to 12 % faster than 4 or 6)
     static_assert(WARP_BYTES % 16 == 0, "16-byte aligned regions");
 };
 
@@ -320,6 +346,7 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
 {
     using F = Fpw<G>;
     constexpr int NS = F::NS, RW = FPW_WARP_RAYS;
+    constexpr int NP = (NS + 1) / 2, V = NS < 4 ? NS : 4;   // pairs of slices a thread sums; slices in one access
     extern __shared__ float4 wsm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     char* region = reinterpret_cast<char*>(wsm) + warp * F::WARP_BYTES;
@@ -348,11 +375,11 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
 
     const int lp = lane % FPW_LP, pair = lane / FPW_LP;
     const int even = fpw_slice<NS>(lp, pair, 0), odd = fpw_slice<NS>(lp, pair, 1);
-    float2 acc[FPW_RAYS][NS / 2];
+    float2 acc[FPW_RAYS][NP];
 #pragma unroll
     for (int r = 0; r < FPW_RAYS; r++)
 #pragma unroll
-        for (int q = 0; q < NS / 2; q++) acc[r][q] = make_float2(0.f, 0.f);
+        for (int q = 0; q < NP; q++) acc[r][q] = make_float2(0.f, 0.f);
 
     const size_t gvol = (size_t)g * Nz * Nx * G;
     const float* v00 = p.vol + gvol + (size_t)(Nz - 1) * Nx * G;   // voxel (0, 0)
@@ -471,24 +498,24 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
                 const float *ve = v + even, *vo = v + odd;
                 const int cols = s_cnt[j];
                 // (the next column is loaded ahead; past the last one it reads on within the warp's region)
-                float2 wt = w[0], a[NS / 2];
+                float2 wt = w[0], a[NP];
                 fpw_load<NS>(ve, vo, a);
 #pragma unroll 2
                 for (int e = 0; e < cols; e++) {
                     ve += G;
                     vo += G;
                     const float2 wn = w[e + 1];
-                    float2 an[NS / 2];
+                    float2 an[NP];
                     fpw_load<NS>(ve, vo, an);
                     const float2 w0 = make_float2(wt.x, wt.x), w1 = make_float2(wt.y, wt.y);
 #pragma unroll
-                    for (int q = 0; q < NS / 2; q++) {
+                    for (int q = 0; q < NP; q++) {
                         fma2(acc[0][q], w0, a[q]);
                         fma2(acc[1][q], w1, a[q]);
                     }
                     wt = wn;
 #pragma unroll
-                    for (int q = 0; q < NS / 2; q++) a[q] = an[q];
+                    for (int q = 0; q < NP; q++) a[q] = an[q];
                 }
                 __syncwarp();   // the stage is free: fetch the row `lead` ahead into the next free stage
                 const int jf = j + lead;
@@ -510,7 +537,7 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
 #pragma unroll
                 for (int r = 0; r < FPW_RAYS; r++)
 #pragma unroll
-                    for (int q = 0; q < NS / 2; q++) acc[r][q] = make_float2(0.f, 0.f);
+                    for (int q = 0; q < NP; q++) acc[r][q] = make_float2(0.f, 0.f);
                 break;
             }
             row = next;
@@ -532,11 +559,11 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
 #pragma unroll
                 for (int m = 0; m < 4; m++) {
                     const float* vm = v + (m & 1) * G - (ptrdiff_t)(m >> 1) * Nx * G;
-                    float2 a[NS / 2];
+                    float2 a[NP];
                     fpw_load<NS>(vm + even, vm + odd, a);
                     const float2 w2 = make_float2(wt[m], wt[m]);
 #pragma unroll
-                    for (int q = 0; q < NS / 2; q++) fma2(acc[r][q], w2, a[q]);
+                    for (int q = 0; q < NP; q++) fma2(acc[r][q], w2, a[q]);
                 }
             }
         }
@@ -548,14 +575,18 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
         const size_t pitch = (size_t)groups * p.nt * N * G;
         float* mine = p.part + (((size_t)g * p.nt + tb) * N + u0) * G;
         auto at = [&](int sg, int r, int b) {
-            return reinterpret_cast<float4*>(mine + sg * pitch + (size_t)(FPW_RAYS * pair + r) * G + fpw_slice<NS>(lp, pair, b));
+            return reinterpret_cast<VecOf<V>*>(mine + sg * pitch + (size_t)(FPW_RAYS * pair + r) * G + fpw_slice<NS>(lp, pair, b));
         };
 #pragma unroll
         for (int r = 0; r < FPW_RAYS; r++)
             if (u0 + FPW_RAYS * pair + r < N) {
 #pragma unroll
-                for (int b = 0; b < NS / 4; b++)
-                    *at(seg, r, b) = make_float4(acc[r][2 * b].x, acc[r][2 * b].y, acc[r][2 * b + 1].x, acc[r][2 * b + 1].y);
+                for (int b = 0; b < NS / V; b++) {
+                    float v[V];
+#pragma unroll
+                    for (int q = 0; q < V; q++) v[q] = q & 1 ? acc[r][(V * b + q) / 2].y : acc[r][(V * b + q) / 2].x;
+                    *at(seg, r, b) = pack<V>(v);
+                }
             }
         __threadfence();
         __syncwarp();
@@ -570,17 +601,22 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
 #pragma unroll
         for (int r = 0; r < FPW_RAYS; r++)
 #pragma unroll
-            for (int q = 0; q < NS / 2; q++) acc[r][q] = make_float2(0.f, 0.f);
+            for (int q = 0; q < NP; q++) acc[r][q] = make_float2(0.f, 0.f);
 #pragma unroll 2
         for (int sg = seg0; sg < seg0 + nseg; sg++)
 #pragma unroll
             for (int r = 0; r < FPW_RAYS; r++)
                 if (u0 + FPW_RAYS * pair + r < N) {
 #pragma unroll
-                    for (int b = 0; b < NS / 4; b++) {
-                        const float4 v = __ldcg(at(sg, r, b));
-                        acc[r][2 * b].x += v.x; acc[r][2 * b].y += v.y;
-                        acc[r][2 * b + 1].x += v.z; acc[r][2 * b + 1].y += v.w;
+                    for (int b = 0; b < NS / V; b++) {
+                        float v[V];
+                        unpack<V>(__ldcg(at(sg, r, b)), v);
+#pragma unroll
+                        for (int q = 0; q < V; q++) {
+                            float2& s2 = acc[r][(V * b + q) / 2];
+                            if (q & 1) s2.y += v[q];
+                            else s2.x += v[q];
+                        }
                     }
                 }
     }
@@ -588,16 +624,16 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
     // mean along the ray, residual and R-factor sums
     float ad = 0.f, ar = 0.f;
     unsigned tested = 0, quads = 0;   // slices summed sample by sample; quads of the group that hold some
-    int ys[NS / 4];
+    int ys[NS / V];
 #pragma unroll
-    for (int k = 0; k < NS / 4; k++) {
+    for (int k = 0; k < NS / V; k++) {
         ys[k] = g * G + fpw_slice<NS>(lp, pair, k);
-        const int4 f = __ldg(reinterpret_cast<const int4*>(p.flags + ys[k]));
-        const int fl[4] = {f.x, f.y, f.z, f.w};
+        float fl[V];
+        unpack<V>(__ldg(reinterpret_cast<const VecOf<V>*>(p.flags + ys[k])), fl);
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-            if (fl[q] & (kFlagVolEmpty | kFlagRawSpecial | kFlagVolSpecial)) {
-                tested |= 1u << (4 * k + q);
+        for (int q = 0; q < V; q++)
+            if (__float_as_int(fl[q]) & (kFlagVolEmpty | kFlagRawSpecial | kFlagVolSpecial)) {
+                tested |= 1u << (V * k + q);
                 quads |= 1u << ((ys[k] - g * G) / 4);
             }
     }
@@ -612,19 +648,18 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
         if (u >= N) continue;
         const float n = (float)max(hi - lo + 1, 0);
 #pragma unroll
-        for (int b = 0; b < NS / 4; b++) {
+        for (int b = 0; b < NS / V; b++) {
             const size_t o = (((size_t)g * p.T + t) * N + u) * G + (ys[b] - g * G);
-            const float4 rw4 = *reinterpret_cast<const float4*>(p.raw + o);
-            const float rw[4] = {rw4.x, rw4.y, rw4.z, rw4.w};
-            const float sums[4] = {acc[r][2 * b].x, acc[r][2 * b].y, acc[r][2 * b + 1].x, acc[r][2 * b + 1].y};
-            float d[4];
+            float rw[V], d[V];
+            unpack<V>(*reinterpret_cast<const VecOf<V>*>(p.raw + o), rw);
             const TestedQuad* tq = res + 2 * k * (G / 4) + (ys[b] - g * G) / 4;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                float sum = sums[q], cnt = n;
-                if ((tested >> (4 * b + q)) & 1) {
-                    sum = tq[0].s[q] + tq[G / 4].s[q];
-                    cnt = tq[0].n[q] + tq[G / 4].n[q];
+            for (int q = 0; q < V; q++) {
+                float sum = q & 1 ? acc[r][(V * b + q) / 2].y : acc[r][(V * b + q) / 2].x, cnt = n;
+                if ((tested >> (V * b + q)) & 1) {
+                    const int e = V == 4 ? q : (ys[b] + q) & 3;
+                    sum = tq[0].s[e] + tq[G / 4].s[e];
+                    cnt = tq[0].n[e] + tq[G / 4].n[e];
                 }
                 const float fp = cnt <= 0.f ? kSentinelValue : sum / cnt;
                 d[q] = 0.f;
@@ -636,7 +671,7 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
                     if (!(fabsf(d[q]) < kSpecial)) atomicOr(p.flags + ys[b] + q, kFlagDiffSpecial);
                 }
             }
-            *reinterpret_cast<float4*>(p.diff + o) = make_float4(d[0], d[1], d[2], d[3]);
+            *reinterpret_cast<VecOf<V>*>(p.diff + o) = pack<V>(d);
         }
     }
     if (p.rf) {
@@ -711,7 +746,7 @@ __device__ __noinline__ TestedQuad bpw_quad_tested(const float* row0, size_t til
 // volume rows of the tile, which arrive while the tilts are summed.
 constexpr int BPW_CHUNK = 3;
 template <int LP>
-__host__ __device__ constexpr int bpw_window() { return LP == 8 ? 22 : 38; }   // |(TX - 1, TZ - 1)| + 6 samples
+__host__ __device__ constexpr int bpw_window() { return LP == 8 ? 22 : LP == 4 ? 38 : LP == 2 ? 70 : 134; }   // |(TX - 1, TZ - 1)| + 6 samples
 template <int LP, int NS>
 __host__ __device__ constexpr size_t bpw_smem()
 {

@@ -143,3 +143,28 @@ def test_sizes_around_the_grid_limits(nx, nz, T):
     assert not seen & 16
     ref = sart(np.ascontiguousarray(f[:, 4:6]), tilts, nz, 0, T, 1, 3, threads=1)
     assert rel_l2(vol[4:6], ref) < max(nz, T) * 2.0 ** -25
+
+
+# walks in one piece and in segments; tilts past the blocked windows; rows with NaN
+@pytest.mark.parametrize("nx,ny,nz,lim,bad", [(140, 64, 37, 60, None), (250, 30, 75, 85, None), (97, 91, 200, 78, None),
+                                              (140, 30, 130, 60, np.nan), (64, 32, 50, 60, np.inf)])
+def test_slabs_of_a_few_slices_give_the_same_bits(nx, ny, nz, lim, bad):
+    """Groups of 4 and 8 slices, which only slabs take, and their workspace."""
+    from aretomo3_b200 import recon
+    tilts = np.linspace(-lim, lim, 21).astype(np.float32)
+    f = _series(nx, ny, tilts, nz, seed=6)
+    if bad is not None:
+        f[3, 5, 30:33] = bad
+    ref, _ = _run(f, tilts, nz, iterations=2, subsets=3)
+    for slab in (1, 3, 4, 6, 8, 9):
+        vol, seen = _run(f, tilts, nz, iterations=2, subsets=3, slab_slices=slab)
+        assert not seen & 16
+        assert np.array_equal(vol, ref, equal_nan=True), slab
+    ws = []
+    for slab in (4, 16):
+        plan = recon.Plan(nx, ny, tilts, nz, method=recon.SART, iterations=2, subsets=3, slab_slices=slab)
+        ws.append(plan.workspace_bytes)
+        assert plan.workspace_bytes <= recon.estimate_bytes(nx, ny, tilts, nz, method=recon.SART, iterations=2, subsets=3,
+                                                            slab_slices=slab)
+        plan.close()
+    assert ws[0] < 0.3 * ws[1]
