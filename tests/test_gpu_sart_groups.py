@@ -168,3 +168,26 @@ def test_slabs_of_a_few_slices_give_the_same_bits(nx, ny, nz, lim, bad):
                                                             slab_slices=slab)
         plan.close()
     assert ws[0] < 0.3 * ws[1]
+
+
+@pytest.mark.parametrize("nx,ny,nz,start,num,subsets", [(130, 32, 40, 3, 17, 4), (96, 64, 130, 0, 23, 5), (65, 30, 31, 7, 9, 9),
+                                                        (48, 50, 20, 22, 1, 2)])
+def test_tilt_range_and_rfactor(nx, ny, nz, start, num, subsets):
+    """Subsets of a part of the tilts (all of them in the first back-projection; a subset may be
+    empty), and the residual sums of each iteration: N * num * ny terms in FP32 warp sums
+    added up in FP64, each with the error of its voxels."""
+    from aretomo3_b200 import recon
+    tilts = np.linspace(-60, 60, 23).astype(np.float32)
+    f = _series(nx, ny, tilts, nz, seed=nx + ny)
+    plan = recon.Plan(nx, ny, tilts, nz, method=recon.SART, start_tilt=start, num_tilts=num, iterations=3, subsets=subsets,
+                      compute_rfactor=True, fill_seed=3)
+    try:
+        vol = np.empty(plan.volume_shape, np.float32)
+        plan.run_host([f[t] for t in range(tilts.size)], [vol[y] for y in range(ny)])
+        rf = plan.rfactor()
+        assert not plan.flags_seen() & 16
+    finally:
+        plan.close()
+    ref, rref = sart(f, tilts, nz, start, num, 3, subsets, rfactor=True)
+    assert rel_l2(vol, ref) < TOL
+    assert np.allclose(rf, rref, rtol=1e-4)
