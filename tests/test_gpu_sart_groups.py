@@ -191,3 +191,65 @@ def test_tilt_range_and_rfactor(nx, ny, nz, start, num, subsets):
     ref, rref = sart(f, tilts, nz, start, num, 3, subsets, rfactor=True)
     assert rel_l2(vol, ref) < TOL
     assert np.allclose(rf, rref, rtol=1e-4)
+
+
+def test_same_bits_captured_served_tuned_and_side_by_side():
+    """A graph of several plans replayed twice, the serving loop with slabs and a tail, a tuned
+    slab, and two plans on two threads and streams: each as the plan alone."""
+    import threading
+
+    import torch
+    from aretomo3_b200 import recon
+    kw = dict(method=recon.SART, iterations=2, subsets=4, fill_seed=3)
+    shapes = [(140, 64, 37, 21), (96, 32, 130, 25), (250, 91, 60, 19)]
+    tl = [np.linspace(-60, 60, T).astype(np.float32) for *_, T in shapes]
+    fr = [_series(nx, ny, t, nz, seed=nx) for (nx, ny, nz, _), t in zip(shapes, tl)]
+    dev = [torch.from_numpy(f).cuda() for f in fr]
+    plans = [recon.Plan(nx, ny, t, nz, **kw) for (nx, ny, nz, _), t in zip(shapes, tl)]
+    vols = [torch.empty(p.volume_shape, device="cuda") for p in plans]
+    ref = []
+    for p, f, v in zip(plans, dev, vols):
+        p.run_device(f.data_ptr(), v.data_ptr(), 0)
+        torch.cuda.synchronize()
+        ref.append(v.cpu().numpy())
+
+    def check(what):
+        torch.cuda.synchronize()
+        for v, r in zip(vols, ref):
+            assert np.array_equal(v.cpu().numpy(), r), what
+            v.fill_(float("nan"))
+        torch.cuda.synchronize()
+
+    check("alone")
+    batch = recon.Batch(plans, [f.data_ptr() for f in dev], [v.data_ptr() for v in vols], branches=2)
+    for _ in range(2):
+        batch.run(torch.cuda.current_stream().cuda_stream)
+        check("captured")
+    batch.close()
+
+    def many(i, stream):
+        for _ in range(4):
+            plans[i].run_device(dev[i].data_ptr(), vols[i].data_ptr(), stream.cuda_stream)
+
+    st = [torch.cuda.Stream() for _ in plans]
+    th = [threading.Thread(target=many, args=(i, st[i])) for i in range(len(plans))]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    check("side by side")
+    plans[2].autotune(dev[2].data_ptr(), vols[2].data_ptr(), 0)
+    for p, f, v in zip(plans, dev, vols):
+        p.run_device(f.data_ptr(), v.data_ptr(), 0)
+    check("tuned")
+    srv = recon.Server(max_inflight=3)
+    try:
+        ids = [srv.submit(f, t, nz, slab_slices=s, **kw)
+               for f, t, (_, _, nz, _), s in list(zip(fr, tl, shapes, (0, 0, 0))) + list(zip(fr, tl, shapes, (20, 5, 33)))]
+        for rid, r in zip(ids, ref + ref):
+            assert np.array_equal(srv.wait(rid)[0], r), "served"
+    finally:
+        srv.close()
+    assert not any(p.flags_seen() & 16 for p in plans)
+    for p in plans:
+        p.close()
