@@ -229,7 +229,6 @@ int bp_window(int tx, int tz, double scale, const std::vector<float>& cs, int T)
     return (int)std::ceil(span) + 6;
 }
 
-// tilts are staged in chunks, so the window buffer does not grow with the tilt count
 // Threads of a row / column FFT launch: 1024 when two CTAs' shared memory
 // would not fit one SM (so one CTA holds 32 warps) and the radix set allows.
 int fft_threads(int rs, size_t smem)
@@ -338,7 +337,7 @@ at3r_status run_sart_wide(at3r_plan* p, const float* proj, size_t tilt_stride, i
     b.sino = dif; b.relax = p->relax; b.low_bit = kFlagDiffLow;
     FpwArgs f{};
     f.vol = w; f.raw = raw; f.diff = dif; f.cs = p->d_cs; f.flags = p->d_flags;
-    f.Nx = Nx; f.Nz = Nz; f.S = S; f.T = T; f.N = N;
+    f.Nx = Nx; f.Nz = Nz; f.T = T; f.N = N;
     f.part = p->d_part; f.arrived = p->d_arrived; f.seg_rows = p->fp_seg_rows;
     f.polls = p->wait_polls;
     const int blocks = (N + FPW_CTA_RAYS - 1) / FPW_CTA_RAYS, segs = (Nz + f.seg_rows - 1) / f.seg_rows;
@@ -608,11 +607,14 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
 at3r_status at3r_plan_create(const at3r_geom* g, at3r_plan** out) { return plan_create_impl(g, nullptr, out); }
 
 // SART on slice groups (sart_wide.cuh): FP32 series whose rows fill the groups.  Full
-// groups take 0.62 (4096 wide) to 0.72 (1024 wide) of the four-slice kernels' time, so they
-// pay as long as filling up costs less than 1.3; the 16-bit forms of the four-slice kernels
-// are as fast as full groups (2048 x 96 x 600: 55.9 ms against 54.7; 925 x 131 x 221:
-// 15.5 against 17.1) and stay.  It follows the series, not the slab, so that a slab size
-// never changes a result.
+// groups take 0.61 (4096 wide) to 0.71 (1024 wide) of the four-slice kernels' time, so they
+// pay as long as filling up costs less than 1.3.  It follows the series, not the slab, so that a
+// slab size never changes a result.  16-bit storage stays on the four-slice kernels, which
+// read a 16-bit volume copy: the forms tried on slice groups were compared only where rows
+// part-fill the groups (2048 x 96 x 600 in three groups of 32: 54.7 ms against 55.9; 925 x 131 x
+// 221 filled up to 160: 17.1 against 15.5), so where they fill groups of 64 the better kernel
+// for them is not known; there FP32 is the faster storage (4096 x 4096 x 41 x 1200, GVoxel*tilt/s:
+// FP32 82.5, FP16 72.9, BF16 70.0).
 constexpr double kWideFill = 1.3;
 // Their grids have the volume rows and the tilts in y; longer series keep the four-slice kernels.
 constexpr int kWideMaxY = 65535;

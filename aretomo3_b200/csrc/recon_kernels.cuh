@@ -167,7 +167,11 @@ __device__ __forceinline__ float row_scale(float absmax) { return absmax > 0.f ?
 constexpr int kFlagVolEmpty = 1;    // the volume holds a -1e30 voxel (AreTomo's "empty")
 constexpr int kFlagRawLow = 2;      // the staged sinogram holds values <= kLowValue
 constexpr int kFlagDiffLow = 4;     // the residual holds values <= kLowValue
-constexpr int kFlagRawSpecial = 32, kFlagDiffSpecial = 64, kFlagVolSpecial = 128;   // see sart_wide.cuh
+// The slice's staged rows, residual or volume hold a value beyond +-1e30, an infinity or a
+// NaN: the blocked sums (sart_wide.cuh, wbp_bp.cuh) multiply neighbouring samples by zero weights,
+// so such a slice takes the per-sample paths.  One bit per producer, so that no kernel tests a
+// bit that it sets itself.
+constexpr int kFlagRawSpecial = 32, kFlagDiffSpecial = 64, kFlagVolSpecial = 128;
 constexpr int kFlagsReported = 31;  // the bits of the run summary
 constexpr float kSpecial = 1e30f;   // values beyond it, infinities and NaN: kFlag*Special
 constexpr float kLowValue = -5.0e9f;  // far from any lerp of values above it reaching -1e10

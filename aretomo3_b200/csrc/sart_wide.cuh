@@ -11,8 +11,8 @@
 // few neighbouring rays or voxels loads the taps they share once.  What a slice's
 // result is made of does not depend on G, so every G gives the same bits.
 // Measured (B200, ms in the two projectors, four-slice kernels first): 4096 x 64 x 41 x
-// 1200, 15 iterations, forward 184 -> 101, back 84 -> 68; 1024 x 256 x 61 x 300,
-// 15 iterations, 64 -> 44 and 31 -> 23.  FP32 only: with a 16-bit copy of the volume the
+// 1200, 15 iterations, forward 184 -> 103, back 84 -> 61; 1024 x 256 x 61 x 300,
+// 15 iterations, 64 -> 45 and 31 -> 22.  FP32 only: with a 16-bit copy of the volume the
 // forward projector's conversions took what the bytes saved (2048 x 96 x 41 x
 // 600, 10 iterations: 33.6 ms against 31.3 for the four-slice 16-bit kernel).
 #pragma once
@@ -22,16 +22,11 @@
 
 namespace at3r {
 
-// Slices whose staged rows, residual or volume hold a value beyond +-1e30, an
-// infinity or a NaN: the blocked sums below multiply neighbouring samples by
-// zero weights, so such a slice takes the per-sample paths.  One bit per
-// producer, so that no kernel tests a bit that it sets itself.
-
 constexpr int WIDE_THREADS = 256, WIDE_WARPS = WIDE_THREADS / 32;
 constexpr int FPW_RAYS = 2;                  // rays a thread carries
 constexpr int FPW_LP = 4;                    // lanes that share its rays
 constexpr int FPW_WARP_RAYS = FPW_RAYS * 32 / FPW_LP, FPW_PAIRS = 32 / FPW_LP;
-constexpr int FPW_MAX_COLS = 32;             // columns of a ray pair's window; wider (steeper than ~83 degrees): per sample
+constexpr int FPW_MAX_COLS = 32;             // columns of a ray pair's window; wider: sample by sample
 constexpr int FPW_MAX_ROWS = 8;              // volume rows per weight table
 constexpr int WIDE_POLLS = 1 << 22;          // polls of a wait for a bulk copy before it gives up
 
@@ -197,8 +192,11 @@ __device__ __forceinline__ void fpw_load(const float* even, const float* odd, fl
 // samples and their validity are the reference's (fp_ray_setup), every value is
 // FP32, and a column that a ray does not touch has weight zero.
 // The window of the warp's rays in a row is one contiguous run of the volume:
-// lane 0 fetches it with one bulk asynchronous copy into a ring of rows, ahead of
-// their use.  A warp shares nothing with the others of its CTA, so no
+// the lane that holds the row's bounds fetches it with one bulk asynchronous copy into a
+// ring of rows, ahead of their use.  The ring holds 80 columns, which the window of 16 rays
+// exceeds from about 77 degrees on (in volumes wider than that); such tilts go sample by sample,
+// one warp for the whole ray, and so do those whose pair window exceeds FPW_MAX_COLS
+// (about 84 degrees).  A warp shares nothing with the others of its CTA, so no
 // block-wide barrier is needed and short rays leave no one waiting.
 // The rows are cut into segments of seg_rows, one warp each: the segments that a ray
 // block crosses leave their sums in `part`, and the last of them to finish adds
@@ -218,7 +216,7 @@ struct FpwArgs {
     float* part;             // ray sums of the segments [segment][group][nt][N][G]
     int* arrived;            // [group][nt][ray warps]: segments done; zero between launches
     int seg_rows;            // volume rows a warp walks
-    int Nx, Nz, S, T, N, t0, nt;
+    int Nx, Nz, T, N, t0, nt;
     int polls;               // limit of a wait for a bulk copy (WIDE_POLLS)
 };
 
@@ -693,8 +691,10 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
 // positions lie within cos + |sin| <= 1.42 of one another, so four consecutive
 // samples hold all their taps, and voxel v takes sample k with the hat weight
 // max(0, 1 - |x_v - k|) — the lerp's own two weights, zero elsewhere.  Four loads
-// of NS slices serve four voxels (eight one voxel at a time).  Rows come from
-// L1 / L2: the CTA's window (16 c + 8 |s| + 4 samples a tilt) is small.
+// of NS slices serve four voxels (eight one voxel at a time).  The CTA's windows
+// (16 c + 8 |s| + 4 samples a tilt) come to shared memory by bulk copies, three tilts
+// ahead (below).  Bound by the multiply-adds: pipe 64 % busy, issue 67 %, shared-memory wavefronts
+// 54 %; the volume read and written once is 47 % of its time at the copy rate.
 // Positions are the reference's FP32 ones and sums run in its (tilt) order.
 // Grid (x tiles, z tiles, groups).
 // ---------------------------------------------------------------------------

@@ -15,9 +15,10 @@
 // index and weights are formed once for the WB slices; sums run in the reference's
 // (tilt) order with packed multiply-adds.
 // Measured (4096 x 128 rows x 41, thickness 1200): 31.6 ms with a pair of samples a voxel
-// (two shared wavefronts a voxel and slice, the LSU path at 76 %) -> 19.1 ms; 512 x 512 x
-// 41 x 128: 1.82 -> 1.12 ms; the FP16 form, which staged half-precision values and
-// differences, 1440 x 512 x 51 x 400: 16.9 -> 15.2 ms with half the error.
+// (two shared wavefronts a voxel and slice, the LSU path at 76 %) -> 18.8 ms; 512 x 512 x
+// 41 x 128: 1.82 -> 1.06 ms; the FP16 form, which staged half-precision values and
+// differences, 1440 x 512 x 51 x 400: 16.9 -> 13.1 ms with half the error.  Bound by the
+// multiply-adds (FMA pipe 72-77 % busy, issue 66 %, shared-memory wavefronts 57 %).
 // Slices whose sinogram holds values near the -1e10 "empty" marker, infinities or
 // NaN (flag bits) are summed sample by sample as the reference tests them.
 #pragma once

@@ -193,7 +193,8 @@ def profiled_traffic(kernel: str, workload_name: str, storage: str):
     return d.get(f"{workload_name}/{storage}", {}).get(kernel)
 
 
-# Shared-memory bytes one work unit of a kernel moves on chip.  WBP back-
+# Shared-memory bytes one work unit of a kernel moves on chip (FP32 SART: of the kernels
+# on slice groups, which the rows of every SART workload here fill).  WBP back-
 # projection: three samples of a slice per block of four voxels.  FP32 SART: four
 # samples per block of four voxels; the forward projector reads, per ray
 # sample and slice, (1 + 2 sin + 2 cos) / 2 columns of a ray pair's window (1.8 on
