@@ -4,8 +4,8 @@
 // voxel or a ray serve all slices.  Here the slices are the innermost index:
 //   volume    W[group][Nz][Nx][G]   rows z flipped, G slices of a group
 //   sinogram  R[group][T][N][G]     weighted rows and residual
-// with G = 16, 32 or 64 (slabs of fewer slices: 8 or 4): a few lanes share a position and carry its G slices, read
-// as contiguous runs.  Every load is then fully coalesced whatever the tilt (with
+// with G = 16, 32 or 64 (slabs of fewer slices: 8 or 4): a few lanes share a position and
+// carry its G slices, read as contiguous runs.  Every load is then fully coalesced whatever the tilt (with
 // rays or voxels on the lanes, a warp's samples lie 1/cos or cos apart and a
 // 16-byte tap load took 6.6 to 8.1 wavefronts for 4), and a thread that carries a
 // few neighbouring rays or voxels loads the taps they share once.  What a slice's
@@ -195,8 +195,7 @@ __device__ __forceinline__ void fpw_load(const float* even, const float* odd, fl
 // the lane that holds the row's bounds fetches it with one bulk asynchronous copy into a
 // ring of rows, ahead of their use.  The ring holds 80 columns, which the window of 16 rays
 // exceeds from about 77 degrees on (in volumes wider than that); such tilts go sample by sample,
-// one warp for the whole ray, and so do those whose pair window exceeds FPW_MAX_COLS
-// (about 84 degrees).  A warp shares nothing with the others of its CTA, so no
+// and so do those whose pair window exceeds FPW_MAX_COLS (about 84 degrees).  A warp shares nothing with the others of its CTA, so no
 // block-wide barrier is needed and short rays leave no one waiting.
 // The rows are cut into segments of seg_rows, one warp each: the segments that a ray
 // block crosses leave their sums in `part`, and the last of them to finish adds
@@ -384,14 +383,12 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
     const int C = fpw_cols(FPW_RAYS - 1, c, s, N, Nx), W = min(Nx, fpw_cols(RW - 1, c, s, N, Nx) + 2);
     const uint32_t row_bytes = (uint32_t)(W * G * sizeof(float));
     const bool blocked = C <= FPW_MAX_COLS && row_bytes <= F::RING;
-    // segments that take part: those the rays cross (one if none, or sample by sample)
-    const int seg = blockIdx.y, seg0 = z1 < z0 || !blocked ? 0 : z0 / p.seg_rows;
-    const int nseg = z1 < z0 || !blocked ? 1 : z1 / p.seg_rows - seg0 + 1;
+    // segments that take part: those the rays cross (one if none)
+    const int seg = blockIdx.y, seg0 = z1 < z0 ? 0 : z0 / p.seg_rows;
+    const int nseg = z1 < z0 ? 1 : z1 / p.seg_rows - seg0 + 1;
     if (seg < seg0 || seg >= seg0 + nseg) return;
-    if (blocked) {
-        z0 = max(z0, seg * p.seg_rows);
-        z1 = min(z1, (seg + 1) * p.seg_rows - 1);
-    }
+    z0 = max(z0, seg * p.seg_rows);
+    z1 = min(z1, (seg + 1) * p.seg_rows - 1);
     if (blocked && z1 >= z0) {
         const int ns = min(FPW_MAX_STAGES, (int)(F::RING / row_bytes));
         if (lane == 0) {
@@ -540,13 +537,16 @@ __global__ void __launch_bounds__(FPW_THREADS, Fpw<G>::CTAS) k_fp_wide(FpwArgs p
             }
             row = next;
         }
-    } else {
-        // steep tilts: sample by sample
+    } else if (!blocked) {
+        // steep tilts: sample by sample, a segment the samples whose lower row it holds
+        const float Z0 = (float)(seg * p.seg_rows), Z1 = (float)((seg + 1) * p.seg_rows);
+        const int slo = first_true(rlo, rhi, est_index(ceilf(__fmaf_rn(Z0 - tz, inv_c, halfL))), [&](int i) { return zpos(i) >= Z0; });
+        const int shi = first_true(slo, rhi, est_index(ceilf(__fmaf_rn(Z1 - tz, inv_c, halfL))), [&](int i) { return zpos(i) >= Z1; }) - 1;
 #pragma unroll
         for (int r = 0; r < FPW_RAYS; r++) {
             const int k = FPW_RAYS * pair + r;
             const float tx = __shfl_sync(0xffffffffu, ray.tx, k);
-            const int lo = __shfl_sync(0xffffffffu, rlo, k), hi = __shfl_sync(0xffffffffu, rhi, k);
+            const int lo = __shfl_sync(0xffffffffu, slo, k), hi = __shfl_sync(0xffffffffu, shi, k);
             for (int i = lo; i <= hi; i++) {
                 const float fd = (float)i - halfL;
                 const float fX = __fmaf_rn(-fd, s, tx), fZ = __fmaf_rn(fd, c, tz);
