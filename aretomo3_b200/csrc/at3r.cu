@@ -618,27 +618,40 @@ at3r_status at3r_plan_create(const at3r_geom* g, at3r_plan** out) { return plan_
 constexpr double kWideFill = 1.3;
 // Their grids have the volume rows and the tilts in y; longer series keep the four-slice kernels.
 constexpr int kWideMaxY = 65535;
-static bool sart_wide(const at3r_geom* g)
-{
-    return g->method == AT3R_SART && g->storage == AT3R_STORE_F32 && wide_cost(g->ny, 16) <= kWideFill * g->ny &&
-           g->vol_z <= kWideMaxY && g->n_tilts <= kWideMaxY;
-}
-
+// Thin volumes keep them too unless the rays of a subset fill the GPU several times over: a launch
+// then takes as long as one walk, whose set-up costs more here (8 iterations, 13 subsets, 128 x 64 x
+// 41 tilts, ms on the four-slice and on these kernels: thickness 8 1.56 and 2.60, 24 2.28 and
+// 2.92, 32 2.63 and 2.89, 40 2.86 and 2.90, 64 3.68 and 2.99; thickness 8, 1 subset, 512 x 64 (1.3 M rays) 0.41 and 0.51,
+// 512 x 256 (5.4 M) 1.02 and 0.86).
+constexpr int kWideThin = 32;
+constexpr long kWideThinRays = 1L << 22;
 // The most tilts of a subset.
 static size_t wide_subset(const at3r_geom* g)
 {
     return std::max(1, (g->num_tilts + g->subsets - 1) / std::max(1, g->subsets));
 }
+static bool sart_wide(const at3r_geom* g)
+{
+    return g->method == AT3R_SART && g->storage == AT3R_STORE_F32 && wide_cost(g->ny, 16) <= kWideFill * g->ny &&
+           g->vol_z <= kWideMaxY && g->n_tilts <= kWideMaxY &&
+           (g->vol_z >= kWideThin || (long)(g->nx & ~1) * g->ny * (long)wide_subset(g) >= kWideThinRays);
+}
+
 // Volume rows per warp of the forward projection: enough segments that one
-// subset's projection gives every SM two rounds of its eight warps, and at most
+// subset's projection gives every SM two rounds of its eight warps (of 24 rows or more), and at most
 // 320 rows, so that the concurrent walks stay within what L2 holds of the
-// volume.  It follows the series, not the slab (the segments' sums are part of a result).
+// volume.  Where one round holds them, up to twelve segments of eight rows or more: the launch takes as
+// long as one walk, about 0.6 us a row (8 iterations, 13 subsets, 128 x 64 x 41 tilts, thickness 40, ms for
+// one segment, three and five: 4.39, 3.16, 2.90; the four-slice kernels 2.86).  It follows the series,
+// not the slab (the segments' sums are part of a result).
 static int wide_seg_rows(const at3r_geom* g)
 {
     // (at least one ray: the size estimates are asked about widths that no plan accepts)
     const long N = std::max(g->nx & ~1, 2), warps = (N + 15) / 16 * (long)wide_subset(g) * ((g->ny + 63) / 64);
-    const long segs = std::max((long)(g->vol_z + 319) / 320, std::min((long)(2 * 8 * 148 + warps - 1) / warps, (long)g->vol_z / 24));
-    return (int)((g->vol_z + std::max(segs, 1L) - 1) / std::max(segs, 1L));
+    const long round = 8 * 148, two = std::min((2 * round + warps - 1) / warps, (long)g->vol_z / 24);
+    const long one = std::min(std::min(round / warps, (long)g->vol_z / 8), 12L);
+    const long segs = std::max(std::max((long)(g->vol_z + 319) / 320, two), std::max(one, 1L));
+    return (int)((g->vol_z + segs - 1) / segs);
 }
 // Counters of the segments: one per group of four or more slices, tilt and 16 rays.
 static size_t wide_arrived(const at3r_geom* g, int slices)
