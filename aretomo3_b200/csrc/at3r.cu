@@ -607,14 +607,14 @@ at3r_status plan_create_impl(const at3r_geom* g, cudaStream_t alloc_stream, at3r
 at3r_status at3r_plan_create(const at3r_geom* g, at3r_plan** out) { return plan_create_impl(g, nullptr, out); }
 
 // SART on slice groups (sart_wide.cuh): FP32 series whose rows fill the groups.  Full
-// groups take 0.61 (4096 wide) to 0.71 (1024 wide) of the four-slice kernels' time, so they
+// groups take 0.60 (4096 wide) to 0.69 (1024 wide) of the four-slice kernels' time, so they
 // pay as long as filling up costs less than 1.3.  It follows the series, not the slab, so that a
 // slab size never changes a result.  16-bit storage stays on the four-slice kernels, which
 // read a 16-bit volume copy: the forms tried on slice groups were compared only where rows
 // part-fill the groups (2048 x 96 x 600 in three groups of 32: 54.7 ms against 55.9; 925 x 131 x
 // 221 filled up to 160: 17.1 against 15.5), so where they fill groups of 64 the better kernel
 // for them is not known; there FP32 is the faster storage (4096 x 4096 x 41 x 1200, GVoxel*tilt/s:
-// FP32 82.5, FP16 72.9, BF16 70.0).
+// FP32 84.5, FP16 72.8, BF16 69.9).
 constexpr double kWideFill = 1.3;
 // Their grids have the volume rows and the tilts in y; longer series keep the four-slice kernels.
 constexpr int kWideMaxY = 65535;

@@ -11,8 +11,8 @@
 // few neighbouring rays or voxels loads the taps they share once.  What a slice's
 // result is made of does not depend on G, so every G gives the same bits.
 // Measured (B200, ms in the two projectors, four-slice kernels first): 4096 x 64 x 41 x
-// 1200, 15 iterations, forward 184 -> 103, back 84 -> 61; 1024 x 256 x 61 x 300,
-// 15 iterations, 64 -> 45 and 31 -> 22.  FP32 only: with a 16-bit copy of the volume the
+// 1200, 15 iterations, forward 184 -> 99, back 84 -> 61; 1024 x 256 x 61 x 300,
+// 15 iterations, 64 -> 43 and 31 -> 22.  FP32 only: with a 16-bit copy of the volume the
 // forward projector's conversions took what the bytes saved (2048 x 96 x 41 x
 // 600, 10 iterations: 33.6 ms against 31.3 for the four-slice 16-bit kernel).
 #pragma once
@@ -247,7 +247,7 @@ struct TestedQuad {
 // waits on L2, which it reads with little reuse (beside the rings, L1 holds a few KB a warp).
 // Measured (forward projections of 2 iterations of 4096 x 64 x 41 x 1200): with a NaN pixel in every
 // row 441 ms one slice at a time, 139 ms, the four-slice kernel 80 ms; in one row 39 and 35
-// ms (32 ms); in none 13.7 ms (25 ms).
+// ms (32 ms); in none 13.2 ms (25 ms).
 constexpr int FPT = 4;
 template <bool EMPTY>
 __device__ __noinline__ TestedQuad fpw_quad_tested(const float* v0, int G, int Nx, RayPos r, int lo, int hi)
